@@ -628,7 +628,7 @@ int32_t enqueue_iteration(fvm_batch *b, bool with_events, int iters) {
       FVM_TRY(b, done(st));
     }
     FVM_TRY(b, mark(K_MON, st));
-    FVM_TRY(b, launch_monitor(Ap, cp, b->prec == FVM_PREC_FP64 ? 1 : 0));
+    FVM_TRY(b, launch_monitor(Ap, cp));
     FVM_TRY(b, done(st));
     return FVM_OK;
   };
@@ -1927,9 +1927,8 @@ extern "C" int32_t fvm_gpu_check_positivity(fvm_handle *h, int32_t *bad_point) {
 extern "C" int32_t fvm_gpu_clcd(fvm_handle *h, double *cl, double *cd) {
   if (!h) return FVM_ERR_ARG;
   fvm_batch *b = h->b;
-  const int serial = b->prec == FVM_PREC_FP64;
-  if (b->prec == FVM_PREC_FP64) FVM_TRY(b, launch_clcd(ptrs<double>(b), b->cfg, h->slot, serial));
-  else FVM_TRY(b, launch_clcd(ptrs<float>(b), b->cfg, h->slot, serial));
+  if (b->prec == FVM_PREC_FP64) FVM_TRY(b, launch_clcd(ptrs<double>(b), b->cfg, h->slot));
+  else FVM_TRY(b, launch_clcd(ptrs<float>(b), b->cfg, h->slot));
   b->launches++;
   MeshCtl c;
   int32_t st = get_ctl(b, h->slot, c);

@@ -1660,75 +1660,121 @@ __global__ void __launch_bounds__(kBlockVerts) k_sa(ArenaPtrs<R> A, int stage, i
 // ---------------------------------------------------------------------------
 // End-of-iteration monitor, one CTA per mesh: conres.f (from the block
 // partials), clcd.f, the positivity verdict, RES.DAT history row and the
-// stop test of main.f:42.  FP64 arithmetic; the clcd sum is the serial
-// Fortran chain when serial_clcd is set.
+// stop test of main.f:42.  FP64 arithmetic; with FP64 states the clcd sum is
+// the serial Fortran chain.
 // ---------------------------------------------------------------------------
-// One solid edge's pressure and viscous force (clcd.f:20-40), added to
-// (xf, yf).  FP32 states: the terms from the FP32 values (the edge vector
-// an FP64 difference rounded once), accumulated in FP64.
+// FP32 states: one solid edge's pressure and viscous force (clcd.f:20-40),
+// the terms from the FP32 values (the edge vector an FP64 difference rounded
+// once), accumulated in FP64.
+__device__ __forceinline__ void wall_force(double2 c1, double2 c2, float mu1, float mu2,
+                                           const Grad<float> &g1, const Grad<float> &g2, float p1,
+                                           float p2, double &xf, double &yf) {
+  const float sx = float(c2.y - c1.y), sy = -float(c2.x - c1.x);
+  const float n2b3 = 2.0f / 3.0f;
+  const float txx = 0.5f * (n2b3 * mu1 * (2.0f * g1.qx[1] - g1.qy[2]) +
+                            n2b3 * mu2 * (2.0f * g2.qx[1] - g2.qy[2]));
+  const float txy = 0.5f * (mu1 * (g1.qy[1] + g1.qx[2]) + mu2 * (g2.qy[1] + g2.qx[2]));
+  const float tyy = 0.5f * (n2b3 * mu1 * (2.0f * g1.qy[2] - g1.qx[1]) +
+                            n2b3 * mu2 * (2.0f * g2.qy[2] - g2.qx[1]));
+  const float pp = 0.5f * (p1 + p2);
+  xf += double(pp * sx - txx * sx - txy * sy);
+  yf += double(pp * sy - txy * sx - tyy * sy);
+}
+
+// FP64, the Fortran chain: clcd.f:34-40 adds three terms per solid edge, one
+// after another, so the additions are serial; nothing else is.  All threads
+// form the terms of a tile of edges in shared memory, then one thread per
+// component adds them in edge order while the other warps form the next
+// tile.  Each addition costs one pass through the FP64 pipe (about 32 ns on
+// this GPU, 2 lanes per SM quarter-cycle), which bounds the chain: with the
+// loads and products of every edge inside it the chain took 1.45 ms for 1024
+// edges, k_monitor 1480 us against FORCE_US us now.  mu = 0 (inviscid meshes)
+// makes both viscous terms zero; subtracting zero changes no sum (it never is
+// -0: it starts at +0), so a tile whose viscous terms all are zero adds the
+// pressure terms alone.  NaN terms count as nonzero.
+constexpr int kForceTile = 256;
+struct ForceTile {
+  double t[3][2][kForceTile];   // pressure, then the two viscous terms: x, y
+};
+
 template <typename R>
-__device__ __forceinline__ void wall_force(double2 c1, double2 c2, R mu1, R mu2, const Grad<R> &g1,
-                                           const Grad<R> &g2, R p1, R p2, double &xf,
-                                           double &yf) {
-  if constexpr (sizeof(R) == 4) {
-    const float sx = float(c2.y - c1.y), sy = -float(c2.x - c1.x);
-    const float n2b3 = 2.0f / 3.0f;
-    const float txx = 0.5f * (n2b3 * mu1 * (2.0f * g1.qx[1] - g1.qy[2]) +
-                              n2b3 * mu2 * (2.0f * g2.qx[1] - g2.qy[2]));
-    const float txy = 0.5f * (mu1 * (g1.qy[1] + g1.qx[2]) + mu2 * (g2.qy[1] + g2.qx[2]));
-    const float tyy = 0.5f * (n2b3 * mu1 * (2.0f * g1.qy[2] - g1.qx[1]) +
-                              n2b3 * mu2 * (2.0f * g2.qy[2] - g2.qx[1]));
-    const float pp = 0.5f * (p1 + p2);
-    xf += double(pp * sx - txx * sx - txy * sy);
-    yf += double(pp * sy - txy * sx - tyy * sy);
+__device__ __forceinline__ bool force_terms(const ArenaPtrs<R> &A, const R4<R> *P, int2 nn, int k,
+                                            ForceTile &s) {
+  const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
+  const double dx = c2.x - c1.x, dy = c2.y - c1.y;
+  const double sx = dy, sy = -dx;
+  const double mu1 = double(A.mu[nn.x]), mu2 = double(A.mu[nn.y]);
+  const Grad<R> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
+  const double p1 = double(P[nn.x].w), p2 = double(P[nn.y].w);
+  const double txx1 = 2.0 / 3.0 * mu1 * (2.0 * double(g1.qx[1]) - double(g1.qy[2]));
+  const double txy1 = mu1 * (double(g1.qy[1]) + double(g1.qx[2]));
+  const double tyy1 = 2.0 / 3.0 * mu1 * (2.0 * double(g1.qy[2]) - double(g1.qx[1]));
+  const double txx2 = 2.0 / 3.0 * mu2 * (2.0 * double(g2.qx[1]) - double(g2.qy[2]));
+  const double txy2 = mu2 * (double(g2.qy[1]) + double(g2.qx[2]));
+  const double tyy2 = 2.0 / 3.0 * mu2 * (2.0 * double(g2.qy[2]) - double(g2.qx[1]));
+  const double pp = 0.5 * (p1 + p2);
+  const double txx = 0.5 * (txx1 + txx2);
+  const double txy = 0.5 * (txy1 + txy2);
+  const double tyy = 0.5 * (tyy1 + tyy2);
+  const double bx = txx * sx, cx = txy * sy, by = txy * sx, cy = tyy * sy;
+  s.t[0][0][k] = pp * sx;
+  s.t[0][1][k] = pp * sy;
+  s.t[1][0][k] = bx;
+  s.t[1][1][k] = by;
+  s.t[2][0][k] = cx;
+  s.t[2][1][k] = cy;
+  return bx != 0.0 || cx != 0.0 || by != 0.0 || cy != 0.0;
+}
+
+// Adds a tile's terms to v in edge order; `viscous`: all three of an edge.
+__device__ __forceinline__ double force_chain(const ForceTile &s, int comp, int n, bool viscous,
+                                              double v) {
+  const double *a = s.t[0][comp], *b = s.t[1][comp], *c = s.t[2][comp];
+  if (viscous) {
+#pragma unroll 4
+    for (int k = 0; k < n; k++) v = ((v + a[k]) - b[k]) - c[k];
   } else {
-    const double dx = c2.x - c1.x, dy = c2.y - c1.y;
-    const double sx = dy, sy = -dx;
-    const double txx = 0.5 * (2.0 / 3.0 * mu1 * (2.0 * double(g1.qx[1]) - double(g1.qy[2])) +
-                              2.0 / 3.0 * mu2 * (2.0 * double(g2.qx[1]) - double(g2.qy[2])));
-    const double txy = 0.5 * (mu1 * (double(g1.qy[1]) + double(g1.qx[2])) +
-                              mu2 * (double(g2.qy[1]) + double(g2.qx[2])));
-    const double tyy = 0.5 * (2.0 / 3.0 * mu1 * (2.0 * double(g1.qy[2]) - double(g1.qx[1])) +
-                              2.0 / 3.0 * mu2 * (2.0 * double(g2.qy[2]) - double(g2.qx[1])));
-    const double pp = 0.5 * (double(p1) + double(p2));
-    xf += pp * sx - txx * sx - txy * sy;
-    yf += pp * sy - txy * sx - tyy * sy;
+#pragma unroll 8
+    for (int k = 0; k < n; k++) v = v + a[k];
   }
+  return v;
 }
 
 template <typename R>
 __device__ void clcd_block(const ArenaPtrs<R> &A, const MeshConst &mc, int mesh_phase,
-                           int serial, double &cl, double &cd) {
-  __shared__ double s_x[kMonitorMaxThreads], s_y[kMonitorMaxThreads];
+                           double &cl, double &cd) {
   const R4<R> *P = A.st[mesh_phase];
   double xf = 0.0, yf = 0.0;
-  if (serial) {
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < mc.nsw; i++) {
-        const int2 nn = A.sw_nodes[mc.sw0 + i];
-        const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
-        const double dx = c2.x - c1.x, dy = c2.y - c1.y;
-        const double sx = dy, sy = -dx;
-        const double mu1 = double(A.mu[nn.x]), mu2 = double(A.mu[nn.y]);
-        const Grad<R> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
-        const double p1 = double(P[nn.x].w), p2 = double(P[nn.y].w);
-        const double txx1 = 2.0 / 3.0 * mu1 * (2.0 * double(g1.qx[1]) - double(g1.qy[2]));
-        const double txy1 = mu1 * (double(g1.qy[1]) + double(g1.qx[2]));
-        const double tyy1 = 2.0 / 3.0 * mu1 * (2.0 * double(g1.qy[2]) - double(g1.qx[1]));
-        const double txx2 = 2.0 / 3.0 * mu2 * (2.0 * double(g2.qx[1]) - double(g2.qy[2]));
-        const double txy2 = mu2 * (double(g2.qy[1]) + double(g2.qx[2]));
-        const double tyy2 = 2.0 / 3.0 * mu2 * (2.0 * double(g2.qy[2]) - double(g2.qx[1]));
-        const double pp = 0.5 * (p1 + p2);
-        const double txx = 0.5 * (txx1 + txx2);
-        const double txy = 0.5 * (txy1 + txy2);
-        const double tyy = 0.5 * (tyy1 + tyy2);
-        xf = xf + pp * sx - txx * sx - txy * sy;
-        yf = yf + pp * sy - txy * sx - tyy * sy;
+  if constexpr (sizeof(R) == 8) {
+    __shared__ ForceTile s_f[2];
+    __shared__ double s_v[2];
+    // warp 0 (lanes 0 and 1) adds tile i while the others form tile i + 1
+    const int nt = (mc.nsw + kForceTile - 1) / kForceTile;
+    double v = 0.0;
+    bool some = false;   // of the tile formed last
+    for (int k = threadIdx.x; k < min(mc.nsw, kForceTile); k += blockDim.x)
+      some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + k], k, s_f[0]);
+    for (int i = 0; i < nt; i++) {
+      const bool viscous = __syncthreads_or(some);
+      some = false;
+      if (threadIdx.x < 32) {
+        if (threadIdx.x < 2)
+          v = force_chain(s_f[i & 1], threadIdx.x, min(mc.nsw - i * kForceTile, kForceTile),
+                          viscous, v);
+      } else if (i + 1 < nt) {
+        const int base = (i + 1) * kForceTile, n = min(mc.nsw - base, kForceTile);
+        for (int k = threadIdx.x - 32; k < n; k += blockDim.x - 32)
+          some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + base + k], k, s_f[(i + 1) & 1]);
       }
     }
+    if (threadIdx.x < 2) s_v[threadIdx.x] = v;
+    __syncthreads();
+    xf = s_v[0];
+    yf = s_v[1];
   } else {
     // each thread's edges i, i + blockDim, ... summed in that order, with
     // the loads of four edges issued together per trip
+    __shared__ double s_x[kMonitorMaxThreads], s_y[kMonitorMaxThreads];
     constexpr int kU = 4;
     const int nt = (int)blockDim.x;
     for (int i0 = threadIdx.x; i0 < mc.nsw; i0 += kU * nt) {
@@ -1753,7 +1799,7 @@ __device__ void clcd_block(const ArenaPtrs<R> &A, const MeshConst &mc, int mesh_
 #pragma unroll
       for (int u = 0; u < kU; u++) {
         if (i0 + u * nt >= mc.nsw) break;
-        wall_force<R>(c1[u], c2[u], mu1[u], mu2[u], g1[u], g2[u], p1[u], p2[u], xf, yf);
+        wall_force(c1[u], c2[u], mu1[u], mu2[u], g1[u], g2[u], p1[u], p2[u], xf, yf);
       }
     }
     s_x[threadIdx.x] = xf;
@@ -1825,7 +1871,7 @@ __device__ void conres_block(const ArenaPtrs<R> &A, const MeshConst &mc, double 
 
 // One CTA (256 threads) per mesh slot listed in mesh_list.
 template <typename R>
-__global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A, int serial_clcd) {
+__global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A) {
   const int m = blockIdx.x;
   MeshCtl &ctl = A.ctl[m];
   if (!ctl.active) return;
@@ -1836,7 +1882,7 @@ __global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A, 
   conres_block<R>(A, mc, sum, mx, arg);
   const int newp = (ctl.phase + 1) % 3;
   double cl, cd;
-  clcd_block<R>(A, mc, newp, serial_clcd, cl, cd);
+  clcd_block<R>(A, mc, newp, cl, cd);
   __syncthreads();
   if (threadIdx.x != 0) return;
   ctl.phase = newp;
@@ -1991,7 +2037,7 @@ __global__ void __launch_bounds__(kBlockVerts) k_conres_part(ArenaPtrs<R> A) {
 // conres (first: set fres1) or clcd for one mesh, routine mode.
 template <typename R>
 __global__ void __launch_bounds__(256) k_routine_monitor(ArenaPtrs<R> A, int mesh, int what,
-                                                         int first, int serial_clcd) {
+                                                         int first) {
   MeshCtl &ctl = A.ctl[mesh];
   const MeshConst &mc = A.mc[mesh];
   if (what == 0) {
@@ -2013,7 +2059,7 @@ __global__ void __launch_bounds__(256) k_routine_monitor(ArenaPtrs<R> A, int mes
     ctl.fres = fres / ctl.fres1;
   } else {
     double cl, cd;
-    clcd_block<R>(A, mc, ctl.phase, serial_clcd, cl, cd);
+    clcd_block<R>(A, mc, ctl.phase, cl, cd);
     if (threadIdx.x != 0) return;
     ctl.cl = cl;
     ctl.cd = cd;

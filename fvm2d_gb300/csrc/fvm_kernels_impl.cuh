@@ -169,9 +169,9 @@ inline cudaError_t flux_attributes(size_t f) {
     k_sa<R><<<fit_grid(c, k_sa<R>, sm), kBlockVerts, sm, c.stream>>>(A, stage, routine, c.max_tri);           \
     return cudaGetLastError();                                                             \
   }                                                                                        \
-  cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c, int serial_clcd) {  \
+  cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c) {                   \
     if (A.nslots <= 0) return cudaSuccess;                                                 \
-    k_monitor<R><<<A.nslots, monitor_threads<R>(), 0, c.stream>>>(A, serial_clcd);         \
+    k_monitor<R><<<A.nslots, monitor_threads<R>(), 0, c.stream>>>(A);                      \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_update(const ArenaPtrs<R> &A, const LaunchCfg &c, int irk) {           \
@@ -188,11 +188,11 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_conres(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int first) {\
     k_conres_part<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                             \
-    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 0, first, 0);                    \
+    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 0, first);                       \
     return cudaGetLastError();                                                             \
   }                                                                                        \
-  cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int serial) { \
-    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 1, 0, serial);                   \
+  cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh) {             \
+    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 1, 0);                           \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_gradient_edge(const ArenaPtrs<R> &A, const LaunchCfg &c) {             \

@@ -55,12 +55,12 @@ inline int pipe_stage_count(uint32_t stage_bytes, int groups, int want) {
   cudaError_t launch_sa(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int routine);\
   cudaError_t launch_step(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage);           \
   size_t smem_step(const LaunchCfg &c, R *);                                              \
-  cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c, int serial_clcd); \
+  cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c);                  \
   cudaError_t launch_update(const ArenaPtrs<R> &A, const LaunchCfg &c, int irk);           \
   cudaError_t launch_time_step(const ArenaPtrs<R> &A, const LaunchCfg &c);                 \
   cudaError_t launch_positivity(const ArenaPtrs<R> &A, const LaunchCfg &c);                \
   cudaError_t launch_conres(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int first);\
-  cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int serial);\
+  cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh);            \
   cudaError_t launch_limitgrad(const ArenaPtrs<R> &A, const LaunchCfg &c);                 \
   cudaError_t launch_gradient_edge(const ArenaPtrs<R> &A, const LaunchCfg &c);             \
   cudaError_t launch_shockind(const ArenaPtrs<R> &A, const LaunchCfg &c);                  \
