@@ -126,6 +126,8 @@ struct fvm_batch {
   uint8_t *vflag = nullptr;
   int2 *ve_rng = nullptr, *vt_rng = nullptr, *va_rng = nullptr;
   uint16_t *ve_list = nullptr, *vt_list = nullptr;
+  int *ve_src = nullptr, *blk_neo = nullptr;   // FP64
+  void *eflux = nullptr, *bflux = nullptr;   // FP64: fluxes of owned edge and boundary entries
   int *va_list = nullptr;
   float2 *va_w = nullptr;   // FP32: Green-Gauss stencil weights per va_list entry
   double *va_dsl = nullptr; // |ds| of each va_list entry's edge
@@ -164,7 +166,8 @@ struct fvm_batch {
   double t_ms[K_COUNT] = {0};
   int64_t t_launch[K_COUNT] = {0};
   int64_t launches = 0;           // kernels launched since creation
-  int kernels_per_iter = 0;
+  int kernels_per_iter = 0;       // timed steps of an iteration
+  int launches_per_iter = 0;      // kernels of an iteration
   cudaStream_t upload = nullptr;      // side stream of deferred admissions
   bool pending = false;               // staged slots wait for batch_commit
   double *dstage = nullptr;           // device staging of driver-order state transfers
@@ -228,6 +231,10 @@ ArenaPtrs<R> ptrs(const fvm_batch *b) {
   A.vflag = b->vflag;
   A.ve_rng = b->ve_rng;
   A.ve_list = b->ve_list;
+  A.ve_src = b->ve_src;
+  A.blk_neo = b->blk_neo;
+  A.eflux = static_cast<R4<R> *>(b->eflux);
+  A.bflux = static_cast<R4<R> *>(b->bflux);
   A.vt_rng = b->vt_rng;
   A.vt_list = b->vt_list;
   A.blocks = b->blocks;
@@ -559,6 +566,9 @@ int32_t batch_commit(fvm_batch *b) {
   return update_work(b);
 }
 
+// Kernels of a flux pass: edges and gather in FP64, one in FP32.
+int flux_kernels(const fvm_batch *b) { return b->prec == FVM_PREC_FP64 ? 2 : 1; }
+
 // kernels of `iters` iterations, in order; optional timing events around
 // each (one iteration only)
 template <typename R>
@@ -566,7 +576,7 @@ int32_t enqueue_iteration(fvm_batch *b, bool with_events, int iters) {
   const ArenaPtrs<R> A = ptrs<R>(b);
   const LaunchCfg &c = b->cfg;
   const bool visc = c.viscous;   // a viscous mesh is resident
-  int k = 0;
+  int k = 0, launched = 0;
   // per-kernel timing events, recorded on the kernel's own stream
   auto mark = [&](int kind, cudaStream_t st) -> cudaError_t {
     if (!with_events) return cudaSuccess;
@@ -574,7 +584,8 @@ int32_t enqueue_iteration(fvm_batch *b, bool with_events, int iters) {
     b->ev_kind[k] = kind;
     return cudaEventRecordWithFlags(b->ev[2 * k], st, cudaEventRecordExternal);
   };
-  auto done = [&](cudaStream_t st) -> cudaError_t {
+  auto done = [&](cudaStream_t st, int kernels = 1) -> cudaError_t {
+    launched += kernels;
     if (!with_events) {
       k++;
       return cudaSuccess;
@@ -608,11 +619,11 @@ int32_t enqueue_iteration(fvm_batch *b, bool with_events, int iters) {
         FVM_TRY(b, mark(K_GRAD, st));
         // inviscid meshes take their time step in the stage-1 gradient pass
         FVM_TRY(b, launch_grad(Ap, cp, s, s == 1 ? 1 : 0, 0));
-        FVM_TRY(b, done(st));
+        FVM_TRY(b, done(st, cp.stencil && cp.any_inviscid && cp.viscous ? 2 : 1));
         if (s == 1 && fork) FVM_TRY(b, cudaEventRecord(fork, st));
         FVM_TRY(b, mark(K_FLUX, st));
         FVM_TRY(b, launch_flux(Ap, cp, s, 1 /*MODE_UPDATE*/, s, 0));
-        FVM_TRY(b, done(st));
+        FVM_TRY(b, done(st, flux_kernels(b)));
       }
       if (s == 1 && fork && b->fused) FVM_TRY(b, cudaEventRecord(fork, st));
     }
@@ -660,6 +671,7 @@ int32_t enqueue_iteration(fvm_batch *b, bool with_events, int iters) {
     }
   }
   b->kernels_per_iter = k / iters;
+  b->launches_per_iter = launched / iters;
   return FVM_OK;
 }
 
@@ -814,7 +826,13 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
   TRYB(dalloc(O, &b->hl_ptr, (size_t)b->cap[P_HP]));
   TRYB(dalloc(O, &b->hl_list, (size_t)b->cap[P_HL]));
   TRYB(dalloc(O, &b->be_ds, (size_t)c.edge_entries));
-  if (precision == FVM_PREC_FP64) TRYB(dalloc(O, &b->be_csl, (size_t)c.edge_entries));
+  if (precision == FVM_PREC_FP64) {
+    TRYB(dalloc(O, &b->be_csl, (size_t)c.edge_entries));
+    TRYB(dalloc(O, &b->ve_src, (size_t)c.edge_incidence));
+    TRYB(dalloc(O, &b->blk_neo, (size_t)c.blocks));
+    TRYB(dalloc(O, (unsigned char **)&b->eflux, 4 * r * (size_t)c.edge_entries));
+    TRYB(dalloc(O, (unsigned char **)&b->bflux, 8 * r * (size_t)c.boundary_entries));
+  }
   TRYB(dalloc(O, &b->bb_nodes, (size_t)c.boundary_entries));
   TRYB(dalloc(O, &b->bt_nodes, (size_t)c.tri_entries));
   TRYB(dalloc(O, &b->elarea, (size_t)c.triangles));
@@ -932,7 +950,7 @@ extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m, f
   fvm_prepared *P = new (std::nothrow) fvm_prepared();
   if (!P) return FVM_ERR_NOMEM;
   P->par = *par;
-  int32_t st = build_layout(*m, kBlockVerts, P->L);
+  int32_t st = build_layout(*m, kBlockVerts, par->precision == FVM_PREC_FP64, P->L);
   if (st != FVM_OK) {
     delete P;
     return st;
@@ -1066,9 +1084,9 @@ extern "C" int64_t fvm_prepared_bytes(const fvm_prepared *prep, int32_t precisio
   const int64_t r = precision == FVM_PREC_FP64 ? 8 : 4;
   const int64_t V = L.np;
   int64_t bytes = V * (3 * 4 * r + 8 * r + 4 * r + 4 * r + 5 * r + 16 + 4 * 8 + 4 + 1 + 3 * 8);
-  bytes += (int64_t)L.be_nodes.size() * (8 + 16 + (r == 4 ? 16 : 32));
-  bytes += (int64_t)L.bb_nodes.size() * 16 + (int64_t)L.bt_nodes.size() * (16 + (r == 4 ? 32 : 0));
-  bytes += (int64_t)L.nt * 8 + (int64_t)L.ve_list.size() * 2 + (int64_t)L.vt_list.size() * 2;
+  bytes += (int64_t)L.be_nodes.size() * (8 + 16 + (r == 4 ? 16 : 64));
+  bytes += (int64_t)L.bb_nodes.size() * (r == 4 ? 16 : 80) + (int64_t)L.bt_nodes.size() * (16 + (r == 4 ? 32 : 0));
+  bytes += (int64_t)L.nt * 8 + (int64_t)L.ve_list.size() * (r == 4 ? 2 : 6) + (int64_t)L.vt_list.size() * 2;
   bytes += (int64_t)L.va_list.size() * (12 + (r == 4 ? 8 : 0)) + (int64_t)L.sw_nodes.size() * 8;
   bytes += (int64_t)L.nblk * (sizeof(BlockInfo) + sizeof(BlockPartial) + 4);
   bytes += (int64_t)L.be_loc.size() * 4 + (int64_t)L.halo_ids.size() * 4;
@@ -1143,6 +1161,11 @@ static int32_t add_prepared(fvm_batch *b, fvm_prepared *prep, int32_t *slot_out,
   for (int &x : halo) x += v0;
   std::vector<int> hlp(L.hl_ptr);
   for (int &x : hlp) x += (int)S.off[P_HL];
+  std::vector<int> vsrc;
+  if (b->ve_src) {
+    vsrc = L.ve_src;
+    for (int &x : vsrc) x += x >= 0 ? (int)S.off[P_BE] : -2 * (int)S.off[P_BB];
+  }
   std::vector<int2> be(L.be_nodes);
   for (int2 &q : be) {
     q.x += v0;
@@ -1216,6 +1239,8 @@ static int32_t add_prepared(fvm_batch *b, fvm_prepared *prep, int32_t *slot_out,
   PUT(put_range(b, b->vt_rng, v0, vt, us));
   PUT(put_range(b, b->va_rng, v0, va, us));
   PUT(put_range(b, b->ve_list, S.off[P_VE], L.ve_list, us));
+  if (b->ve_src) PUT(put_range(b, b->ve_src, S.off[P_VE], vsrc, us));
+  if (b->blk_neo) PUT(put_range(b, b->blk_neo, S.off[P_BLK], L.neo, us));
   PUT(put_range(b, b->vt_list, S.off[P_VT], L.vt_list, us));
   PUT(put_range(b, b->va_list, S.off[P_VA], valist, us));
   PUT(put_range(b, b->blocks, S.off[P_BLK], blocks, us));
@@ -1391,14 +1416,14 @@ extern "C" int32_t fvm_batch_step(fvm_batch *b, int32_t niter) {
     if ((st = build_graph(b, kGraphIters))) return st;
     for (; niter >= kGraphIters; niter -= kGraphIters) {
       FVM_TRY(b, cudaGraphLaunch(b->graph_multi, b->stream));
-      b->launches += (int64_t)b->kernels_per_iter * kGraphIters;
+      b->launches += (int64_t)b->launches_per_iter * kGraphIters;
     }
   }
   if (niter == 0) return FVM_OK;
   if ((st = build_graph(b, 1))) return st;
   for (int i = 0; i < niter; i++) {
     FVM_TRY(b, cudaGraphLaunch(b->graph, b->stream));
-    b->launches += b->kernels_per_iter;
+    b->launches += b->launches_per_iter;
     if (b->timing) {
       FVM_TRY(b, cudaStreamSynchronize(b->stream));
       for (int k = 0; k < b->kernels_per_iter; k++) {
@@ -1660,7 +1685,7 @@ extern "C" int32_t fvm_batch_test_wait_timeout(fvm_batch *b, int64_t budget_cycl
 extern "C" int32_t fvm_layout_stats(const fvm_mesh *m, int64_t *out) {
   if (!m || !out) return FVM_ERR_ARG;
   MeshLayout L;
-  int32_t st = build_layout(*m, kBlockVerts, L);
+  int32_t st = build_layout(*m, kBlockVerts, true, L);
   if (st) return st;
   out[0] = L.nblk;
   out[1] = (int64_t)L.be_nodes.size();
@@ -1696,7 +1721,7 @@ int32_t residu_impl(fvm_handle *h) {
   if (h->iflow != FVM_INVISCID) FVM_TRY(b, launch_visc(A, b->cfg, 0, 0, 1));
   FVM_TRY(b, launch_grad(A, b->cfg, 0, 0, 1));
   FVM_TRY(b, launch_flux(A, b->cfg, 0, 0 /*MODE_RESIDUAL*/, 0, 1));
-  b->launches += (h->iflow != FVM_INVISCID) ? 3 : 2;
+  b->launches += (h->iflow != FVM_INVISCID) + 1 + flux_kernels(b);
   FVM_TRY(b, cudaStreamSynchronize(b->stream));
   return FVM_OK;
 }
@@ -1736,7 +1761,7 @@ extern "C" int32_t fvm_gpu_create(const fvm_params *par, const fvm_mesh *m, fvm_
   MeshLayout L;
   if (!m->edge || !m->iedge || !m->elem || !m->ptype || (m->nbe > 0 && !m->beindx))
     return FVM_ERR_ARG;
-  int32_t st = build_layout(*m, kBlockVerts, L);
+  int32_t st = build_layout(*m, kBlockVerts, true, L);
   if (st) return st;
   fvm_batch_caps c;
   std::memset(&c, 0, sizeof(c));

@@ -18,6 +18,8 @@
 //     phase 2  each vertex sums its edge fluxes in original iedge order,
 //              then solid and farfield contributions in beindx order, then
 //              applies the RK stage and writes the next state buffer.
+//   FP64 batches run the two phases as two kernels with the fluxes in a
+//   global buffer, every edge computed once, by the block that owns it.
 //
 // Summation order per vertex equals the Fortran serial order, so the FP64
 // build (no FMA contraction) reproduces the reference arithmetic exactly.
@@ -234,6 +236,7 @@ struct ArenaPtrs {
   // incidence: per vertex {begin, end} into the list arrays
   const int2 *ve_rng;
   const uint16_t *ve_list;
+  const int *ve_src;      // FP64: per incidence, its flux: eflux[x], or bflux[-1 - x] of a boundary edge
   const int2 *vt_rng;
   const uint16_t *vt_list;
   // block entries
@@ -242,6 +245,9 @@ struct ArenaPtrs {
   const int2 *be_nodes;   // interior edge entries (n1, n2)
   const double2 *be_ds;   // ds of the edge (flength.f:38-39)
   const D4 *be_csl;       // (ct, st, length) precomputed in FP64
+  const int *blk_neo;     // FP64: entries [e0, e0 + neo) a block (index: its part) owns
+  R4<R> *eflux;           // FP64: interior flux of each owned edge entry
+  R4<R> *bflux;           // FP64: each boundary entry's contributions to n1, n2
   const int4 *bb_nodes;   // boundary entries (n1, n2, type, -)
   const int4 *bt_nodes;   // triangle entries (n1, n2, n3, arena triangle)
   const double *elarea;   // per arena triangle

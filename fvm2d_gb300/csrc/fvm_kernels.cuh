@@ -1031,51 +1031,79 @@ __device__ __forceinline__ void edge_flux(const ArenaPtrs<R> &A, const FluxConst
   }
 }
 
-// Phase 1b of the flux pass: boundary edges, two slots each (contribution
-// to n1, to n2) after the block's ne interior slots.
+// One boundary edge: its contributions to n1 and n2.
+template <typename R>
+__device__ __forceinline__ void boundary_flux(const ArenaPtrs<R> &A, const MeshConst &mc,
+                                              const MeshCtl &ctl, int4 b, const R4<R> *P,
+                                              R4<R> &o1, R4<R> &o2) {
+  const double2 x1 = A.coord[b.x], x2 = A.coord[b.y];
+  const R4<R> p1 = P[b.x], p2 = P[b.y];
+  if (b.z == 1) {
+    // solid_flux.f:10-17
+    const R sx = R(0.5) * R(x2.y - x1.y);
+    const R sy = -R(0.5) * R(x2.x - x1.x);
+    const R pp1 = R(0.75) * p1.w + R(0.25) * p2.w;
+    const R pp2 = R(0.25) * p1.w + R(0.75) * p2.w;
+    o1.x = R(0);
+    o1.y = pp1 * sx;
+    o1.z = pp1 * sy;
+    o1.w = R(0);
+    o2.x = R(0);
+    o2.y = pp2 * sx;
+    o2.z = pp2 * sy;
+    o2.w = R(0);
+  } else {
+    R f1[4], f2[4];
+    farfield_flux<R>(mc, ctl.cl, x1, x2, p1, p2, f1, f2);
+    o1.x = f1[0];
+    o1.y = f1[1];
+    o1.z = f1[2];
+    o1.w = f1[3];
+    o2.x = f2[0];
+    o2.y = f2[1];
+    o2.z = f2[2];
+    o2.w = f2[3];
+  }
+}
+
+// Phase 1b of the FP32 flux pass: boundary edges, two slots each
+// (contribution to n1, to n2) after the block's ne interior slots.
 template <typename R>
 __device__ __forceinline__ void flux_boundary(const ArenaPtrs<R> &A, const MeshConst &mc,
                                               const MeshCtl &ctl, const BlockInfo &bi,
                                               const R4<R> *P, R4<R> *s_flux) {
   for (int k = threadIdx.x; k < bi.nb; k += blockDim.x) {
-    const int4 b = A.bb_nodes[bi.b0 + k];
-    const double2 x1 = A.coord[b.x], x2 = A.coord[b.y];
-    const R4<R> p1 = P[b.x], p2 = P[b.y];
     R4<R> o1, o2;
-    if (b.z == 1) {
-      // solid_flux.f:10-17
-      const R sx = R(0.5) * R(x2.y - x1.y);
-      const R sy = -R(0.5) * R(x2.x - x1.x);
-      const R pp1 = R(0.75) * p1.w + R(0.25) * p2.w;
-      const R pp2 = R(0.25) * p1.w + R(0.75) * p2.w;
-      o1.x = R(0);
-      o1.y = pp1 * sx;
-      o1.z = pp1 * sy;
-      o1.w = R(0);
-      o2.x = R(0);
-      o2.y = pp2 * sx;
-      o2.z = pp2 * sy;
-      o2.w = R(0);
-    } else {
-      R f1[4], f2[4];
-      farfield_flux<R>(mc, ctl.cl, x1, x2, p1, p2, f1, f2);
-      o1.x = f1[0];
-      o1.y = f1[1];
-      o1.z = f1[2];
-      o1.w = f1[3];
-      o2.x = f2[0];
-      o2.y = f2[1];
-      o2.z = f2[2];
-      o2.w = f2[3];
-    }
+    boundary_flux<R>(A, mc, ctl, A.bb_nodes[bi.b0 + k], P, o1, o2);
     s_flux[bi.ne + 2 * k] = o1;
     s_flux[bi.ne + 2 * k + 1] = o2;
   }
 }
 
-// Phase 2 of the flux pass: one thread per vertex sums its edge slots in
+// Adds one incidence's flux to a vertex's residual.
+template <typename R>
+__device__ __forceinline__ void add_flux(R acc[4], uint16_t e, const R4<R> &f) {
+  if (e & kSolidBit) {
+    acc[1] = acc[1] + f.y;
+    acc[2] = acc[2] + f.z;
+  } else if (e & kNegBit) {
+    acc[0] = acc[0] - f.x;
+    acc[1] = acc[1] - f.y;
+    acc[2] = acc[2] - f.z;
+    acc[3] = acc[3] - f.w;
+  } else {
+    acc[0] = acc[0] + f.x;
+    acc[1] = acc[1] + f.y;
+    acc[2] = acc[2] + f.z;
+    acc[3] = acc[3] + f.w;
+  }
+}
+
+// Phase 2 of the flux pass: one thread per vertex sums its edge fluxes in
 // Fortran order, then writes the residual (MODE_RESIDUAL) or applies the RK
 // stage (MODE_UPDATE); at stage 3 the block's conres partial follows.
+// FP32: the fluxes are the block's slots in shared memory (s_flux); FP64:
+// the entries of the global buffers the edge pass filled.
 template <typename R>
 __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshConst &mc,
                                             MeshCtl &ctl, const BlockInfo &bi, const R4<R> *P,
@@ -1098,36 +1126,30 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
       acc[0] = acc[1] = acc[2] = acc[3] = R(0);
     }
     const int2 jr = A.ve_rng[v];
-    // FVM_GATHER_BATCH incidences' slots and fluxes loaded together, then
-    // added in list order
-    constexpr int GB = sizeof(R) == 4 ? FVM_GATHER_BATCH : 1;
+    // GB incidences' slots and fluxes loaded together, then added in list
+    // order (FP64: the loads reach L2, four hide their latency)
+    constexpr int GB = sizeof(R) == 4 ? FVM_GATHER_BATCH : 4;
     for (int j = jr.x; j < jr.y; j += GB) {
       uint16_t es[GB];
       R4<R> fs[GB];
 #pragma unroll
       for (int u = 0; u < GB; u++) es[u] = j + u < jr.y ? A.ve_list[j + u] : uint16_t(0);
+      if constexpr (sizeof(R) == 4) {
 #pragma unroll
-      for (int u = 0; u < GB; u++)
-        if (j + u < jr.y) fs[u] = s_flux[es[u] & kSlotMask];
+        for (int u = 0; u < GB; u++)
+          if (j + u < jr.y) fs[u] = s_flux[es[u] & kSlotMask];
+      } else {
+        int src[GB];
+#pragma unroll
+        for (int u = 0; u < GB; u++) src[u] = j + u < jr.y ? A.ve_src[j + u] : 0;
+#pragma unroll
+        for (int u = 0; u < GB; u++)
+          if (j + u < jr.y) fs[u] = src[u] >= 0 ? A.eflux[src[u]] : A.bflux[-1 - src[u]];
+      }
 #pragma unroll
       for (int u = 0; u < GB; u++) {
         if (j + u >= jr.y) break;
-        const uint16_t e = es[u];
-        const R4<R> f = fs[u];
-        if (e & kSolidBit) {
-          acc[1] = acc[1] + f.y;
-          acc[2] = acc[2] + f.z;
-        } else if (e & kNegBit) {
-          acc[0] = acc[0] - f.x;
-          acc[1] = acc[1] - f.y;
-          acc[2] = acc[2] - f.z;
-          acc[3] = acc[3] - f.w;
-        } else {
-          acc[0] = acc[0] + f.x;
-          acc[1] = acc[1] + f.y;
-          acc[2] = acc[2] + f.z;
-          acc[3] = acc[3] + f.w;
-        }
+        add_flux<R>(acc, es[u], fs[u]);
       }
     }
     if (mode == MODE_RESIDUAL) {
@@ -1159,10 +1181,75 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
     block_conres_partial<R>(have, rho_new, rho_old, org, s_red, s_max, s_arg, A.part + bi.part);
 }
 
+// FP64 flux pass, first kernel: the flux of every edge once, into eflux (the
+// entry of the block owning it), and of every boundary edge into bflux.  The
+// FP64 pipe bounds it: 2 lanes per SM and clock against ~430 operations per
+// edge, so nothing may be computed twice and no SM may idle.  One work item
+// is kEdgeThreads owned entries of a block (the last item of a block: its
+// boundary edges), many items per SM.  One kernel over whole blocks computed
+// cut edges in both blocks (+10%) and left most SMs idle in its last wave:
+// 1365 us for 1024 x 384, Roe; now 1000 us here (446 operations per edge at
+// the pipe's 526 Gop/s) and 149 us in the gather.
+constexpr int kEdgeThreads = 128;
 template <typename R, int FLUX>
-__global__ void __launch_bounds__(sizeof(R) == 4 ? kFluxThreads : kBlockVerts,
-                                  sizeof(R) == 4 ? FVM_FLUX_MINB32 : 2)
+__global__ void __launch_bounds__(kEdgeThreads, 4)
+    k_eflux(ArenaPtrs<R> A, int stage, int routine, int items) {
+  static_assert(sizeof(R) == 8, "the FP64 pass");
+  int w0, nwork;
+  work_range(A, w0, nwork);
+  for (int i = w0 * items + blockIdx.x; i < nwork * items; i += gridDim.x) {
+    const BlockInfo &bi = work_block(A, i / items);
+    const int c = i % items;
+    MeshCtl &ctl = A.ctl[bi.mesh];
+    if (!routine && !ctl.active) continue;
+    const MeshConst &mc = A.mc[bi.mesh];
+    const R4<R> *P = A.st[cur_buf(ctl.phase, stage)];
+    if (c == items - 1) {
+      for (int k = threadIdx.x; k < bi.nb; k += kEdgeThreads) {
+        const int b = bi.b0 + k;
+        boundary_flux<R>(A, mc, ctl, A.bb_nodes[b], P, A.bflux[2 * b], A.bflux[2 * b + 1]);
+      }
+      continue;
+    }
+    const int k = c * kEdgeThreads + threadIdx.x;
+    if (k >= A.blk_neo[bi.part]) continue;
+    R f[4];
+    int err = 0;
+    edge_flux<R, FLUX>(A, flux_const<R>(mc), P, bi.e0 + k, f, err);
+    R4<R> o;
+    o.x = f[0];
+    o.y = f[1];
+    o.z = f[2];
+    o.w = f[3];
+    A.eflux[bi.e0 + k] = o;
+    if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
+  }
+}
+
+// FP64 flux pass, second kernel: gather per vertex and RK stage.
+template <typename R>
+__global__ void __launch_bounds__(kBlockVerts, 2)
+    k_egather(ArenaPtrs<R> A, int stage, int mode, int irk, int routine) {
+  __shared__ double s_red[kBlockVerts / 32], s_max[kBlockVerts / 32];
+  __shared__ int s_arg[kBlockVerts / 32];
+  int w0, nwork;
+  work_range(A, w0, nwork);
+  for (int w = w0 + blockIdx.x; w < nwork; w += gridDim.x) {
+    const BlockInfo bi = work_block(A, w);
+    MeshCtl &ctl = A.ctl[bi.mesh];
+    if (!routine && !ctl.active) continue;
+    const int p = ctl.phase;
+    flux_gather<R>(A, A.mc[bi.mesh], ctl, bi, A.st[cur_buf(p, stage)], nullptr, p, stage, mode,
+                   irk, routine, s_red, s_max, s_arg);
+    __syncthreads();   // s_red, s_max, s_arg are free again
+  }
+}
+
+// FP32 flux pass: both phases in one kernel, the fluxes in shared memory.
+template <typename R, int FLUX>
+__global__ void __launch_bounds__(kFluxThreads, FVM_FLUX_MINB32)
     k_flux(ArenaPtrs<R> A, int stage, int mode, int irk, int routine) {
+  static_assert(sizeof(R) == 4, "the FP32 pass");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R4<R> *s_flux = reinterpret_cast<R4<R> *>(smem_raw);
   __shared__ double s_red[kFluxThreads / 32];
@@ -1171,52 +1258,30 @@ __global__ void __launch_bounds__(sizeof(R) == 4 ? kFluxThreads : kBlockVerts,
   int w0, nwork;
   work_range(A, w0, nwork);
   for (int w = w0 + blockIdx.x; w < nwork; w += gridDim.x) {
+    // (an L2 prefetch of the next block's inputs made the pass slower:
+    // 0.206 -> 0.216 ms on 8 meshes of 1024 x 384 timed alone)
     const BlockInfo bi = work_block(A, w);
     MeshCtl &ctl = A.ctl[bi.mesh];
     if (!routine && !ctl.active) continue;
     const MeshConst &mc = A.mc[bi.mesh];
     const int p = ctl.phase;
     const R4<R> *P = A.st[cur_buf(p, stage)];
-    // FP64: the next block's inputs into L2.  Not in FP32, where the same
-    // prefetches made the pass slower (0.206 -> 0.216 ms on 8 meshes of
-    // 1024 x 384 timed alone; whole iterations 1.025 -> 1.040 ms).
-    if (sizeof(R) == 8 && threadIdx.x == 0) {
-      const BlockInfo *nb = next_block(A, w, nwork);
-      if (nb) {
-        const BlockInfo n = *nb;
-        prefetch_l2(A.be_nodes + n.e0, sizeof(int2) * n.ne);
-        prefetch_l2(A.be_csl + n.e0, sizeof(D4) * n.ne);
-        prefetch_l2(P + n.v0, sizeof(R4<R>) * n.nv);
-        prefetch_l2(A.grad + n.v0, sizeof(Grad<R>) * n.nv);
-        prefetch_l2(A.coord + n.v0, sizeof(double2) * n.nv);
-        prefetch_l2(A.ve_rng + n.v0, sizeof(int2) * n.nv);
-        if (mode == MODE_UPDATE) {
-          prefetch_l2(A.st[old_buf(p, stage)] + n.v0, sizeof(R4<R>) * n.nv);
-          prefetch_l2(A.dt + n.v0, sizeof(R) * n.nv);
-          prefetch_l2(A.cvarea + n.v0, sizeof(R) * n.nv);
-        }
-      }
-    }
     int err = 0;
     FluxConst<R> fc;
-    if constexpr (sizeof(R) == 4 && (FLUX & kFluxStd) != 0) fc = flux_const_std(mc);
+    if constexpr ((FLUX & kFluxStd) != 0) fc = flux_const_std(mc);
     else fc = flux_const<R>(mc);
-    // phase 1a: interior edges.  FP32: the next entry's ends are loaded
-    // while this entry's states and gradients are in flight
+    // phase 1a: interior edges; the next entry's ends are loaded while this
+    // entry's states and gradients are in flight
 #if FVM_FLUX_PIPE
     int2 nn_next = make_int2(0, 0);
-    if (sizeof(R) == 4 && threadIdx.x < bi.ne) nn_next = A.be_nodes[bi.e0 + threadIdx.x];
+    if (threadIdx.x < bi.ne) nn_next = A.be_nodes[bi.e0 + threadIdx.x];
 #endif
     for (int k = threadIdx.x; k < bi.ne; k += blockDim.x) {
       R f[4];
 #if FVM_FLUX_PIPE
-      if constexpr (sizeof(R) == 4) {
-        const int2 nn = nn_next;
-        if (k + (int)blockDim.x < bi.ne) nn_next = A.be_nodes[bi.e0 + k + blockDim.x];
-        edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err, &nn);
-      } else {
-        edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err);
-      }
+      const int2 nn = nn_next;
+      if (k + (int)blockDim.x < bi.ne) nn_next = A.be_nodes[bi.e0 + k + blockDim.x];
+      edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err, &nn);
 #else
       edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err);
 #endif

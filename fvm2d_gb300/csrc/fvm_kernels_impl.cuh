@@ -22,48 +22,64 @@ inline int fit_grid(const LaunchCfg &c, K kern, size_t smem, int threads = kBloc
   return g < c.grid ? g : c.grid;
 }
 
-// The flux pass for template code F (Riemann solver | kFluxStd).
+// The flux pass for template code F (Riemann solver | kFluxStd).  FP32: one
+// kernel; FP64: every edge once, then the gather.
 template <typename R, int F>
-inline void launch_flux_code(const ArenaPtrs<R> &A, const LaunchCfg &c, size_t sm, int nt,
-                             int stage, int mode, int irk, int routine) {
-  k_flux<R, F><<<fit_grid(c, k_flux<R, F>, sm, nt), nt, sm, c.stream>>>(A, stage, mode, irk,
-                                                                         routine);
+inline void launch_flux_code(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,
+                             int irk, int routine) {
+  if constexpr (sizeof(R) == 4) {
+    const size_t sm = size_t(c.max_slots) * sizeof(R4<R>);
+    k_flux<R, F><<<fit_grid(c, k_flux<R, F>, sm, kFluxThreads), kFluxThreads, sm, c.stream>>>(
+        A, stage, mode, irk, routine);
+  } else {
+    // a block's owned entries in items of kEdgeThreads, and its boundary edges
+    const int items = (c.max_slots + kEdgeThreads - 1) / kEdgeThreads + 1;
+    LaunchCfg ce = c;
+    ce.grid = c.grid > INT_MAX / items ? INT_MAX : c.grid * items;
+    k_eflux<R, F><<<fit_grid(ce, k_eflux<R, F>, 0, kEdgeThreads), kEdgeThreads, 0, c.stream>>>(
+        A, stage, routine, items);
+    k_egather<R><<<fit_grid(c, k_egather<R>, 0), kBlockVerts, 0, c.stream>>>(A, stage, mode, irk,
+                                                                             routine);
+  }
 }
 template <typename R>
-inline void launch_flux_any(const ArenaPtrs<R> &A, const LaunchCfg &c, size_t sm, int nt,
-                            int stage, int mode, int irk, int routine) {
+inline void launch_flux_any(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,
+                            int irk, int routine) {
   if constexpr (sizeof(R) == 4) {
     if (c.std_const) {
       switch (c.flux) {
-        case 1: launch_flux_code<R, 1 | kFluxStd>(A, c, sm, nt, stage, mode, irk, routine); return;
-        case 2: launch_flux_code<R, 2 | kFluxStd>(A, c, sm, nt, stage, mode, irk, routine); return;
-        case 3: launch_flux_code<R, 3 | kFluxStd>(A, c, sm, nt, stage, mode, irk, routine); return;
-        default: launch_flux_code<R, kFluxStd>(A, c, sm, nt, stage, mode, irk, routine); return;
+        case 1: launch_flux_code<R, 1 | kFluxStd>(A, c, stage, mode, irk, routine); return;
+        case 2: launch_flux_code<R, 2 | kFluxStd>(A, c, stage, mode, irk, routine); return;
+        case 3: launch_flux_code<R, 3 | kFluxStd>(A, c, stage, mode, irk, routine); return;
+        default: launch_flux_code<R, kFluxStd>(A, c, stage, mode, irk, routine); return;
       }
     }
   }
   switch (c.flux) {
-    case 1: launch_flux_code<R, 1>(A, c, sm, nt, stage, mode, irk, routine); return;
-    case 2: launch_flux_code<R, 2>(A, c, sm, nt, stage, mode, irk, routine); return;
-    case 3: launch_flux_code<R, 3>(A, c, sm, nt, stage, mode, irk, routine); return;
-    default: launch_flux_code<R, 0>(A, c, sm, nt, stage, mode, irk, routine); return;
+    case 1: launch_flux_code<R, 1>(A, c, stage, mode, irk, routine); return;
+    case 2: launch_flux_code<R, 2>(A, c, stage, mode, irk, routine); return;
+    case 3: launch_flux_code<R, 3>(A, c, stage, mode, irk, routine); return;
+    default: launch_flux_code<R, 0>(A, c, stage, mode, irk, routine);
   }
 }
-// dynamic shared memory attribute of every flux-pass instantiation
+
+// Dynamic shared memory of the FP32 flux kernels (FP64: none).
 template <typename R>
 inline cudaError_t flux_attributes(size_t f) {
-  const int b = (int)f;
-  cudaError_t e = cudaFuncSetAttribute(k_flux<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
   if constexpr (sizeof(R) == 4) {
+    const int b = (int)f;
+    cudaError_t e = cudaFuncSetAttribute(k_flux<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 1 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 2 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 3 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    return e;
+  } else {
+    return cudaSuccess;
   }
-  return e;
 }
 
 #define FVM_DEFINE_LAUNCHERS(R)                                                            \
@@ -138,10 +154,8 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_flux(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,   \
                           int irk, int routine) {                                          \
-    size_t sm = smem_flux(c, (R *)nullptr);                                                \
-    if (sm > kMaxSmem) return cudaErrorInvalidConfiguration;                              \
-    const int nt = sizeof(R) == 4 ? kFluxThreads : kBlockVerts;                           \
-    launch_flux_any<R>(A, c, sm, nt, stage, mode, irk, routine);                           \
+    if (smem_flux(c, (R *)nullptr) > kMaxSmem) return cudaErrorInvalidConfiguration;       \
+    launch_flux_any<R>(A, c, stage, mode, irk, routine);                                      \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   size_t smem_step(const LaunchCfg &c, R *) {                                              \

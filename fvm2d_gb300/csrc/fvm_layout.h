@@ -20,12 +20,15 @@ struct MeshLayout {
   std::vector<int> iperm;         // driver vertex -> new vertex
   std::vector<BlockInfo> blocks;  // v0,e0,b0,t0 relative; mesh/part filled at upload
   std::vector<int2> be_nodes;     // interior edge entries (new ids)
+  std::vector<int> neo;           // owned_first: per block, its own edges (the first of its entries)
   std::vector<int> be_edge;       // driver edge index (0-based) of each entry
   std::vector<int4> bb_nodes;     // boundary entries (n1, n2, 1 solid | 2 farfield, -)
   std::vector<int4> bt_nodes;     // triangle entries (n1, n2, n3, driver triangle)
   std::vector<uint32_t> bt_loc;   // per triangle entry: the ends' local slots (kTriLoc*)
   std::vector<int> ve_ptr;        // [np+1]
   std::vector<uint16_t> ve_list;
+  std::vector<int> ve_src;        // owned_first: per ve_list entry: the edge's entry in its owner block, or
+                                  // -1 - (2 x boundary entry + end) of a boundary edge
   std::vector<int> vt_ptr;        // [np+1]
   std::vector<uint16_t> vt_list;
   std::vector<int> va_ptr;        // [np+1] all netot edges, edge order
@@ -41,10 +44,11 @@ struct MeshLayout {
   int max_halo = 0;               // max halo vertices of a block
 };
 
-// Builds the layout; returns FVM_OK or FVM_ERR_ARG (bad connectivity) /
+// Builds the layout (owned_first: each block's own edges first in its list,
+// and ve_src, for FP64 batches); returns FVM_OK or FVM_ERR_ARG (bad connectivity) /
 // FVM_ERR_CAPACITY (a block needs more slots than the incidence entries can
 // address).
-int32_t build_layout(const fvm_mesh &m, int block_verts, MeshLayout &L);
+int32_t build_layout(const fvm_mesh &m, int block_verts, bool owned_first, MeshLayout &L);
 
 // Checks the fused-pass invariants of a built layout (local slots decode to
 // the edge ends, halo triangle lists equal the owners' lists in order,
