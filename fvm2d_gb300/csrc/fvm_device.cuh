@@ -14,12 +14,18 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "fvm_ieee64.h"
 #include "fvm_internal.h"
 
 namespace fvm {
 
 __device__ __forceinline__ float msqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double msqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ F64 msqrt(F64 x) { return F64(sqrt64(x.v)); }
+__device__ __forceinline__ F64 merf(F64 x) { return F64(erf(x.v)); }
+__device__ __forceinline__ F64 mexp(F64 x) { return F64(exp(x.v)); }
+__device__ __forceinline__ F64 mpow(F64 x, F64 y) { return F64(pow(x.v, y.v)); }
+__device__ __forceinline__ F64 mdiv(F64 a, F64 b) { return a / b; }
 __device__ __forceinline__ float merf(float x) { return erff(x); }
 __device__ __forceinline__ double merf(double x) { return erf(x); }
 // FP32: the fast hardware approximations (a few ulp), like the approximate
@@ -74,6 +80,23 @@ __device__ __forceinline__ float limit_albada<float>(float ul, float ur, float e
   const float bot = fmaf(ul, ul, fmaf(ur, ur, 2.0f * eps));
   const float r = __fdividef(top, bot);
   return (p <= 0.0f) ? 0.0f : r;
+}
+
+// F64: the sign test of the product needs no product when both operands are
+// inside the window, where it cannot underflow
+template <>
+__device__ __forceinline__ F64 limit_albada<F64>(F64 ul, F64 ur, F64 eps) {
+  const uint32_t a = (uint32_t)__double2hiint(ul.v), b = (uint32_t)__double2hiint(ur.v);
+  const uint32_t ea = (a & 0x7ff00000u) - 0x30000000u, eb = (b & 0x7ff00000u) - 0x30000000u;
+  if (i64_outside(ea | eb)) {
+    if (i64_hw_mul(ul.v, ur.v) <= 0.0) return F64(0.0);
+  } else if ((int)(a ^ b) < 0) {
+    return F64(0.0);
+  }
+  const F64 ul2 = sq(ul), ur2 = sq(ur);
+  const F64 top = (ul2 + eps) * ur + (ur2 + eps) * ul;
+  const F64 bot = ul2 + ur2 + F64(2.0 * eps.v);
+  return top / bot;
 }
 
 // recon.f:4-50 for one variable

@@ -977,58 +977,56 @@ __device__ __forceinline__ void recon_edge_f32(const R4<float> &p1, const R4<flo
 
 // FLUX = 1/2/3 compiles one Riemann solver only (every resident mesh uses
 // it); FLUX = 0 dispatches on the mesh's iflux.
-// nn_in: the entry's ends when the caller has loaded them (FP32 edge loop),
-// else nullptr
-template <typename R, int FLUX>
-__device__ __forceinline__ void edge_flux(const ArenaPtrs<R> &A, const FluxConst<R> &fc,
-                                          const R4<R> *P, int e, R f[4], int &err,
-                                          const int2 *nn_in = nullptr) {
-  int2 nn;
-  R dx, dy, ct, st, len;
-  float dsx = 0.f, dsy = 0.f;
-  if constexpr (sizeof(R) == 4) {
-    // ends, edge vector and ds (24 bytes per entry); ds/|ds| and |ds| are
-    // formed after the reconstruction
-    nn = nn_in ? *nn_in : A.be_nodes[e];
-    const float4 h = A.be_g32[e].v;
-    dx = h.x;
-    dy = h.y;
-    dsx = h.z;
-    dsy = h.w;
-  } else {
-    nn = A.be_nodes[e];
-    const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
-    dx = c2.x - c1.x;
-    dy = c2.y - c1.y;
-  }
-  const R4<R> p1 = P[nn.x], p2 = P[nn.y];
-  const Grad<R> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
-  R pl[4], pr[4];
-  if constexpr (sizeof(R) == 4) {
-    recon_edge_f32(p1, p2, g1, g2, dx, dy, fc, pl, pr);
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      recon1<R>(comp(p1, q), comp(p2, q), g1.qx[q], g1.qy[q], g2.qx[q], g2.qy[q], dx, dy,
-                fc.ilimit, fc.a11, fc.a12, fc.a21, fc.a22, fc.eps, pl[q], pr[q]);
-  }
-  if constexpr (sizeof(R) == 4) {
-    edge_normal_f32(dsx, dsy, ct, st, len);
-  } else {
-    const D4 csl = A.be_csl[e];
-    ct = R(csl.x);
-    st = R(csl.y);
-    len = R(csl.z);
-  }
+template <typename T, int FLUX>
+__device__ __forceinline__ bool riemann(const FluxConst<T> &fc, T ct, T st, T len, const T pl[4],
+                                        const T pr[4], T f[4]) {
   constexpr int FL = FLUX & 3;
   const int which = FL ? FL : fc.iflux;
-  if (which == 1) {
-    if (!roe_flux<R>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, f)) err = 1;
-  } else if (which == 2) {
-    kfvs_flux<R>(ct, st, len, pl, pr, fc.gamma1, fc.pi, f);
+  if (which == 1) return roe_flux<T>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, f);
+  if (which == 2) {
+    kfvs_flux<T>(ct, st, len, pl, pr, fc.gamma1, fc.pi, f);
   } else {
-    hllc_flux<R>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, fc.rotate_back, f);
+    hllc_flux<T>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, fc.rotate_back, f);
   }
+  return true;
+}
+
+// FP32: the flux of edge entry e with ends nn (24 bytes per entry: the ends,
+// edge vector and ds; ds/|ds| and |ds| are formed after the reconstruction)
+template <int FLUX>
+__device__ __forceinline__ void edge_flux_f32(const ArenaPtrs<float> &A, const FluxConst<float> &fc,
+                                              const R4<float> *P, int e, int2 nn, float f[4],
+                                              int &err) {
+  const float4 h = A.be_g32[e].v;
+  const R4<float> p1 = P[nn.x], p2 = P[nn.y];
+  const Grad<float> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
+  float pl[4], pr[4], ct, st, len;
+  recon_edge_f32(p1, p2, g1, g2, h.x, h.y, fc, pl, pr);
+  edge_normal_f32(h.z, h.w, ct, st, len);
+  if (!riemann<float, FLUX>(fc, ct, st, len, pl, pr, f)) err = 1;
+}
+
+// FP64: the flux of edge entry e, products, quotients and roots in integer
+// arithmetic (fvm_ieee64.h)
+template <int FLUX>
+__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<double> &A, const FluxConst<F64> &fc,
+                                              const R4<double> *P, int e, R4<double> &o, int &err) {
+  const int2 nn = A.be_nodes[e];
+  const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
+  const R4<double> p1 = P[nn.x], p2 = P[nn.y];
+  const Grad<double> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
+  const D4 csl = A.be_csl[e];
+  const F64 dx = c2.x - c1.x, dy = c2.y - c1.y;
+  F64 pl[4], pr[4], f[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    recon1<F64>(comp(p1, q), comp(p2, q), g1.qx[q], g1.qy[q], g2.qx[q], g2.qy[q], dx, dy,
+                fc.ilimit, fc.a11, fc.a12, fc.a21, fc.a22, fc.eps, pl[q], pr[q]);
+  if (!riemann<F64, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f)) err = 1;
+  o.x = f[0].v;
+  o.y = f[1].v;
+  o.z = f[2].v;
+  o.w = f[3].v;
 }
 
 // One boundary edge: its contributions to n1 and n2.
@@ -1188,8 +1186,10 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // is kEdgeThreads owned entries of a block (the last item of a block: its
 // boundary edges), many items per SM.  One kernel over whole blocks computed
 // cut edges in both blocks (+10%) and left most SMs idle in its last wave:
-// 1365 us for 1024 x 384, Roe; now 1000 us here (446 operations per edge at
-// the pipe's 526 Gop/s) and 149 us in the gather.
+// 1365 us for 1024 x 384, Roe; 1000 us here (446 operations per edge at the
+// pipe's 526 Gop/s) and 149 us in the gather; with the products, quotients
+// and roots on the integer pipes (F64) 1000 -> 540 us (512 x 192: 261 -> 139;
+// HLLC on 768 x 256: 1064 -> 771, its pow still on the FP64 pipe).
 constexpr int kEdgeThreads = 128;
 template <typename R, int FLUX>
 __global__ void __launch_bounds__(kEdgeThreads, 4)
@@ -1213,14 +1213,9 @@ __global__ void __launch_bounds__(kEdgeThreads, 4)
     }
     const int k = c * kEdgeThreads + threadIdx.x;
     if (k >= A.blk_neo[bi.part]) continue;
-    R f[4];
     int err = 0;
-    edge_flux<R, FLUX>(A, flux_const<R>(mc), P, bi.e0 + k, f, err);
     R4<R> o;
-    o.x = f[0];
-    o.y = f[1];
-    o.z = f[2];
-    o.w = f[3];
+    edge_flux_f64<FLUX>(A, flux_const<F64>(mc), P, bi.e0 + k, o, err);
     A.eflux[bi.e0 + k] = o;
     if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
   }
@@ -1281,10 +1276,10 @@ __global__ void __launch_bounds__(kFluxThreads, FVM_FLUX_MINB32)
 #if FVM_FLUX_PIPE
       const int2 nn = nn_next;
       if (k + (int)blockDim.x < bi.ne) nn_next = A.be_nodes[bi.e0 + k + blockDim.x];
-      edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err, &nn);
 #else
-      edge_flux<R, FLUX>(A, fc, P, bi.e0 + k, f, err);
+      const int2 nn = A.be_nodes[bi.e0 + k];
 #endif
+      edge_flux_f32<FLUX>(A, fc, P, bi.e0 + k, nn, f, err);
       R4<R> o;
       o.x = f[0];
       o.y = f[1];
@@ -1479,14 +1474,7 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_FLUX_MINB32 
         recon1<R>(comp(p1, q), comp(p2, q), g1.qx[q], g1.qy[q], g2.qx[q], g2.qy[q], dx, dy,
                   fc.ilimit, fc.a11, fc.a12, fc.a21, fc.a22, fc.eps, pl[q], pr[q]);
       R f[4];
-      const int which = FLUX ? FLUX : fc.iflux;
-      if (which == 1) {
-        if (!roe_flux<R>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, f)) err = 1;
-      } else if (which == 2) {
-        kfvs_flux<R>(ct, st, len, pl, pr, fc.gamma1, fc.pi, f);
-      } else {
-        hllc_flux<R>(ct, st, len, pl, pr, fc.gamma, fc.gamma1, fc.rotate_back, f);
-      }
+      if (!riemann<R, FLUX>(fc, ct, st, len, pl, pr, f)) err = 1;
       R4<R> o;
       o.x = f[0];
       o.y = f[1];
