@@ -137,7 +137,7 @@ struct fvm_batch {
   double2 *be_ds = nullptr;
   D4 *be_csl = nullptr;
   int4 *bb_nodes = nullptr, *bt_nodes = nullptr;
-  double *elarea = nullptr;
+  double *areat = nullptr;
   EdgeGeo32 *be_g32 = nullptr;
   TriGeo32 *tri_g32 = nullptr;
   uint32_t *be_loc = nullptr;
@@ -244,7 +244,7 @@ ArenaPtrs<R> ptrs(const fvm_batch *b) {
   A.be_csl = b->be_csl;
   A.bb_nodes = b->bb_nodes;
   A.bt_nodes = b->bt_nodes;
-  A.elarea = b->elarea;
+  A.areat = b->areat;
   A.be_g32 = b->be_g32;
   A.tri_g32 = b->tri_g32;
   A.be_loc = b->be_loc;
@@ -835,7 +835,7 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
   }
   TRYB(dalloc(O, &b->bb_nodes, (size_t)c.boundary_entries));
   TRYB(dalloc(O, &b->bt_nodes, (size_t)c.tri_entries));
-  TRYB(dalloc(O, &b->elarea, (size_t)c.triangles));
+  TRYB(dalloc(O, &b->areat, (size_t)c.triangles));
   if (precision == FVM_PREC_FP32) {
     TRYB(dalloc(O, &b->be_g32, (size_t)c.edge_entries));
     TRYB(dalloc(O, &b->va_w, (size_t)c.all_incidence));
@@ -929,7 +929,7 @@ struct fvm_prepared {
   fvm_params par{};
   MeshLayout L;
   std::vector<double2> coord;
-  std::vector<double> ais, cvarea, drmin, wd, elarea;
+  std::vector<double> ais, cvarea, drmin, wd, areat;
   std::vector<int> orig;
   std::vector<double2> be_ds;
   std::vector<EdgeGeo32> be_g32;   // FP32 batches
@@ -938,7 +938,10 @@ struct fvm_prepared {
   std::vector<TriGeo32> tri_g32;   // FP32 batches
 };
 
-extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m, fvm_prepared **out) {
+// fvm_batch_prepare with blocks of at most block_verts vertices (a multiple of
+// kVertAlign, at most kBlockVerts)
+static int32_t prepare_mesh(const fvm_params *par, const fvm_mesh *m, int block_verts,
+                            fvm_prepared **out) {
   if (!par || !m || !out) return FVM_ERR_ARG;
   *out = nullptr;
   if (m->np < 3 || m->nt < 1 || m->netot < 1 || m->ne < 1 || !m->coord || !m->elem ||
@@ -950,7 +953,7 @@ extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m, f
   fvm_prepared *P = new (std::nothrow) fvm_prepared();
   if (!P) return FVM_ERR_NOMEM;
   P->par = *par;
-  int32_t st = build_layout(*m, kBlockVerts, par->precision == FVM_PREC_FP64, P->L);
+  int32_t st = build_layout(*m, block_verts, par->precision == FVM_PREC_FP64, P->L);
   if (st != FVM_OK) {
     delete P;
     return st;
@@ -973,7 +976,8 @@ extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m, f
     if (m->wd) P->wd[v] = m->wd[o];
     P->orig[v] = o + 1;
   }
-  P->elarea.assign(m->elarea, m->elarea + L.nt);
+  P->areat.resize(L.nt);
+  for (int t = 0; t < L.nt; t++) P->areat[t] = 0.25 / m->elarea[t];   // green_gauss.f:180
   P->be_ds.resize(L.be_edge.size());
   P->be_g32.resize(L.be_edge.size());
   for (size_t k = 0; k < L.be_edge.size(); k++) {
@@ -1065,12 +1069,17 @@ extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m, f
     g.dbyy[0] = (float)(x3 - x2);
     g.dbyy[1] = (float)(x1 - x3);
     g.dbyy[2] = (float)(x2 - x1);
-    g.areat = (float)(0.25 / m->elarea[t]);
+    g.areat = (float)P->areat[t];
     g.loc = L.bt_loc[k];
     P->tri_g32[k] = g;
   }
   *out = P;
   return FVM_OK;
+}
+
+extern "C" int32_t fvm_batch_prepare(const fvm_params *par, const fvm_mesh *m,
+                                     fvm_prepared **out) {
+  return prepare_mesh(par, m, kBlockVerts, out);
 }
 
 extern "C" int32_t fvm_prepared_free(fvm_prepared *prep) {
@@ -1254,7 +1263,7 @@ static int32_t add_prepared(fvm_batch *b, fvm_prepared *prep, int32_t *slot_out,
     PUT(launch_edge_csl(b->be_ds + S.off[P_BE], b->be_csl + S.off[P_BE], (int)be.size(), us));
   PUT(put_range(b, b->bb_nodes, S.off[P_BB], bb, us));
   PUT(put_range(b, b->bt_nodes, S.off[P_BT], bt, us));
-  PUT(put_range(b, b->elarea, S.off[P_TRI], prep->elarea, us));
+  PUT(put_range(b, b->areat, S.off[P_TRI], prep->areat, us));
   if (b->be_g32) PUT(put_range(b, b->be_g32, S.off[P_BE], prep->be_g32, us));
   if (b->tri_g32) PUT(put_range(b, b->tri_g32, S.off[P_BT], prep->tri_g32, us));
   if (b->va_w) PUT(put_range(b, b->va_w, S.off[P_VA], prep->va_w, us));
@@ -1712,6 +1721,8 @@ struct fvm_handle {
 
 namespace {
 
+int single_block_verts(int32_t) { return kBlockVerts; }
+
 Slot &hslot(fvm_handle *h) { return h->b->slots[h->slot]; }
 
 template <typename R>
@@ -1757,12 +1768,13 @@ extern "C" int32_t fvm_gpu_create(const fvm_params *par, const fvm_mesh *m, fvm_
   if (!par || !m || !out) return FVM_ERR_ARG;
   *out = nullptr;
   if (m->np < 3 || m->nt < 1) return FVM_ERR_ARG;
-  // size the arena exactly for this mesh
-  MeshLayout L;
   if (!m->edge || !m->iedge || !m->elem || !m->ptype || (m->nbe > 0 && !m->beindx))
     return FVM_ERR_ARG;
-  int32_t st = build_layout(*m, kBlockVerts, true, L);
+  fvm_prepared *prep = nullptr;
+  int32_t st = prepare_mesh(par, m, single_block_verts(m->np), &prep);
   if (st) return st;
+  // the arena exactly for this mesh
+  const MeshLayout &L = prep->L;
   fvm_batch_caps c;
   std::memset(&c, 0, sizeof(c));
   c.vertices = L.np;
@@ -1785,13 +1797,15 @@ extern "C" int32_t fvm_gpu_create(const fvm_params *par, const fvm_mesh *m, fvm_
   c.halo_incidence = std::max<int64_t>(1, L.hl_list.size());
   c.grid = L.nblk;
   fvm_handle *h = new (std::nothrow) fvm_handle();
-  if (!h) return FVM_ERR_NOMEM;
-  if ((st = fvm_batch_create(par->precision, &c, &h->b))) {
-    delete h;
-    return st;
+  if (!h) {
+    fvm_prepared_free(prep);
+    return FVM_ERR_NOMEM;
   }
-  if ((st = fvm_batch_add(h->b, par, m, &h->slot))) {
-    fvm_batch_destroy(h->b);
+  st = fvm_batch_create(par->precision, &c, &h->b);
+  if (!st) st = fvm_batch_add_prepared(h->b, prep, &h->slot);
+  if (st) {
+    fvm_prepared_free(prep);
+    if (h->b) fvm_batch_destroy(h->b);
     delete h;
     return st;
   }

@@ -215,6 +215,15 @@ FVM_I64 double sqrt64(double a) {
   return i64_double((uint32_t)(m0 >> 32) + e, (uint32_t)m0);
 }
 
+// 0.5 a: exact, the exponent less one.  p + 0.5 a: one fused operation, whose
+// product is exact (a subnormal a apart, where half an ulp of 2^-1074 is lost).
+FVM_I64 double half64(double a) {
+  const uint64_t u = i64_bits(a);
+  const uint32_t h = (uint32_t)(u >> 32);
+  if (i64_outside((h & 0x7ff00000u) - 0x30000000u)) return i64_hw_mul(0.5, a);
+  return i64_double(h - 0x00100000u, (uint32_t)u);
+}
+
 // a < 0, a > 0 (false for NaN and zeros)
 FVM_I64 bool neg64(double a) {
   const uint64_t u = i64_bits(a);
@@ -227,7 +236,9 @@ FVM_I64 bool pos64(double a) {
 
 // A double whose products, quotients and square roots are the ones above and
 // whose sums are the FP64 pipe's; the arithmetic of fvm_device.cuh compiles
-// for it as for double.
+// for it as for double.  The / operator calls a function (shorter code: the
+// HLLC flux, which divides 25 times, 639 -> 597 us on 768 x 256), mdiv is
+// inlined.
 struct F64 {
   double v;
   F64() = default;
@@ -238,10 +249,12 @@ FVM_I64 F64 operator+(F64 a, F64 b) { return F64(a.v + b.v); }
 FVM_I64 F64 operator-(F64 a, F64 b) { return F64(a.v - b.v); }
 FVM_I64 F64 operator-(F64 a) { return F64(-a.v); }
 FVM_I64 F64 operator*(F64 a, F64 b) { return F64(mul64(a.v, b.v)); }
-FVM_I64 F64 operator/(F64 a, F64 b) { return F64(div64(a.v, b.v)); }
+FVM_I64_CALL double i64_div_call(double a, double b) { return div64(a, b); }
+FVM_I64 F64 operator/(F64 a, F64 b) { return F64(i64_div_call(a.v, b.v)); }
 FVM_I64 bool operator<(F64 a, F64 b) { return a.v < b.v; }
 FVM_I64 bool operator>(F64 a, F64 b) { return a.v > b.v; }
 FVM_I64 bool operator<=(F64 a, F64 b) { return a.v <= b.v; }
 FVM_I64 bool operator>=(F64 a, F64 b) { return a.v >= b.v; }
+FVM_I64 bool operator!=(F64 a, F64 b) { return a.v != b.v; }
 
 }  // namespace fvm

@@ -250,7 +250,7 @@ struct ArenaPtrs {
   R4<R> *bflux;           // FP64: each boundary entry's contributions to n1, n2
   const int4 *bb_nodes;   // boundary entries (n1, n2, type, -)
   const int4 *bt_nodes;   // triangle entries (n1, n2, n3, arena triangle)
-  const double *elarea;   // per arena triangle
+  const double *areat;    // per arena triangle: 0.25/elarea (green_gauss.f:180)
   const EdgeGeo32 *be_g32; // FP32 path: edge vector and ds of each edge entry (ends: be_nodes)
   const float *ais32, *cvarea32, *drmin32, *wd32;   // FP32 path: per-vertex copies
   const TriGeo32 *tri_g32; // FP32 path: per triangle entry of the blocks (bt_* order)

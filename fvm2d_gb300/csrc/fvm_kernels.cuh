@@ -29,6 +29,9 @@
 #ifndef FVM_STENCIL_MINB
 #define FVM_STENCIL_MINB 6  // resident CTAs per SM asked of the stencil gradient kernel
 #endif
+#ifndef FVM_EFLUX_MINB
+#define FVM_EFLUX_MINB 4    // resident CTAs per SM asked of the FP64 edge kernel (5-8: 3-8% slower)
+#endif
 #ifndef FVM_GATHER_BATCH
 #define FVM_GATHER_BATCH 1  // FP32 flux pass: incidences loaded together in the per-vertex gather
 #endif
@@ -241,6 +244,7 @@ struct TriSmem {
 // a + b rounded as written (never fused with a product that forms b)
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ F64 add_rn(F64 a, F64 b) { return F64(__dadd_rn(a.v, b.v)); }
 
 // Green-Gauss terms of one triangle (green_gauss.f:100-127): dbxx/dbyy of
 // its vertices and the sums dxt/dyt of the four primitive variables.
@@ -286,7 +290,7 @@ struct TriVisc {
 template <typename R>
 __device__ __forceinline__ R tri_areat(const ArenaPtrs<R> &A, const int4 &t, int entry) {
   if constexpr (sizeof(R) == 4) return A.tri_g32[entry].areat;
-  else return 0.25 / A.elarea[t.w];   // green_gauss.f:180
+  else return A.areat[t.w];
 }
 
 template <typename R>
@@ -375,7 +379,7 @@ __device__ __forceinline__ void grad_vertex_sums(const uint16_t *vtl, int j0, in
 }
 
 template <typename R>
-__global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 : 1)
+__global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 : 2)
     k_grad(ArenaPtrs<R> A, int stage, int do_dt,
                                                       int routine, int max_tri, int skip_inviscid) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1006,27 +1010,38 @@ __device__ __forceinline__ void edge_flux_f32(const ArenaPtrs<float> &A, const F
   if (!riemann<float, FLUX>(fc, ct, st, len, pl, pr, f)) err = 1;
 }
 
-// FP64: the flux of edge entry e, products, quotients and roots in integer
-// arithmetic (fvm_ieee64.h)
+// FP64: the flux of edge entry e.  The four variables' reconstructions are one
+// loop, its results in shared memory (`face`: 8 rows of kEdgeThreads, this
+// thread's column): integer arithmetic makes long code, and unrolled the pass
+// waited for instructions a quarter of the time.
+constexpr int kEdgeThreads = 128;
 template <int FLUX>
-__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<double> &A, const FluxConst<F64> &fc,
-                                              const R4<double> *P, int e, R4<double> &o, int &err) {
+__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<F64> &A, const FluxConst<F64> &fc,
+                                              const R4<F64> *P, int e, double *face, F64 f[4],
+                                              int &err) {
   const int2 nn = A.be_nodes[e];
   const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
-  const R4<double> p1 = P[nn.x], p2 = P[nn.y];
-  const Grad<double> g1 = A.grad[nn.x], g2 = A.grad[nn.y];
+  const double dx = c2.x - c1.x, dy = c2.y - c1.y;
+  const double *s1 = reinterpret_cast<const double *>(P + nn.x);
+  const double *s2 = reinterpret_cast<const double *>(P + nn.y);
+  const double *g1 = reinterpret_cast<const double *>(A.grad + nn.x);
+  const double *g2 = reinterpret_cast<const double *>(A.grad + nn.y);
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) {
+    double pl, pr;
+    recon1_f64(s1[q], s2[q], g1[q], g1[4 + q], g2[q], g2[4 + q], dx, dy, fc.ilimit, fc.a11.v,
+               fc.a12.v, fc.a21.v, fc.a22.v, fc.eps.v, pl, pr);
+    face[q * kEdgeThreads] = pl;
+    face[(4 + q) * kEdgeThreads] = pr;
+  }
   const D4 csl = A.be_csl[e];
-  const F64 dx = c2.x - c1.x, dy = c2.y - c1.y;
-  F64 pl[4], pr[4], f[4];
+  F64 pl[4], pr[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++)
-    recon1<F64>(comp(p1, q), comp(p2, q), g1.qx[q], g1.qy[q], g2.qx[q], g2.qy[q], dx, dy,
-                fc.ilimit, fc.a11, fc.a12, fc.a21, fc.a22, fc.eps, pl[q], pr[q]);
+  for (int q = 0; q < 4; q++) {
+    pl[q] = face[q * kEdgeThreads];
+    pr[q] = face[(4 + q) * kEdgeThreads];
+  }
   if (!riemann<F64, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f)) err = 1;
-  o.x = f[0].v;
-  o.y = f[1].v;
-  o.z = f[2].v;
-  o.w = f[3].v;
 }
 
 // One boundary edge: its contributions to n1 and n2.
@@ -1062,6 +1077,28 @@ __device__ __forceinline__ void boundary_flux(const ArenaPtrs<R> &A, const MeshC
     o2.z = f2[2];
     o2.w = f2[3];
   }
+}
+
+// FP64: component `row` of the two contributions of boundary entry b.
+__device__ __forceinline__ void boundary_row(const ArenaPtrs<F64> &A, const MeshConst &mc,
+                                             const MeshCtl &ctl, int b, const R4<F64> *P,
+                                             int row) {
+  const int4 n = A.bb_nodes[b];
+  const double2 x1 = A.coord[n.x], x2 = A.coord[n.y];
+  const R4<F64> p1 = P[n.x], p2 = P[n.y];
+  double f1 = 0.0, f2 = 0.0;
+  if (n.z == 1) {
+    // solid_flux.f:10-17
+    if (row == 1 || row == 2) {
+      const double s = row == 1 ? 0.5 * (x2.y - x1.y) : -0.5 * (x2.x - x1.x);
+      f1 = (0.75 * p1.w.v + 0.25 * p2.w.v) * s;
+      f2 = (0.25 * p1.w.v + 0.75 * p2.w.v) * s;
+    }
+  } else {
+    farfield_row(mc, ctl.cl, x1, x2, p1, p2, row, f1, f2);
+  }
+  reinterpret_cast<double *>(A.bflux + 2 * (size_t)b)[row] = f1;
+  reinterpret_cast<double *>(A.bflux + 2 * (size_t)b + 1)[row] = f2;
 }
 
 // Phase 1b of the FP32 flux pass: boundary edges, two slots each
@@ -1186,15 +1223,17 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // is kEdgeThreads owned entries of a block (the last item of a block: its
 // boundary edges), many items per SM.  One kernel over whole blocks computed
 // cut edges in both blocks (+10%) and left most SMs idle in its last wave:
-// 1365 us for 1024 x 384, Roe; 1000 us here (446 operations per edge at the
-// pipe's 526 Gop/s) and 149 us in the gather; with the products, quotients
-// and roots on the integer pipes (F64) 1000 -> 540 us (512 x 192: 261 -> 139;
-// HLLC on 768 x 256: 1064 -> 771, its pow still on the FP64 pipe).
-constexpr int kEdgeThreads = 128;
+// 1365 us for 1024 x 384, Roe; 1000 us here on the FP64 pipe alone (446
+// operations per edge at 526 Gop/s) and 149 us in the gather; 560 and 103 us
+// with the products, quotients and roots on the integer pipes (F64).  Now
+// neither pipe is full (FP64 57%, ALU 30%, issue 30%): 15 warps per SM wait
+// for each other's results and for instructions.  HLLC on 768 x 256: 1064 ->
+// 597 us, its pow still on the FP64 pipe.
 template <typename R, int FLUX>
-__global__ void __launch_bounds__(kEdgeThreads, 4)
+__global__ void __launch_bounds__(kEdgeThreads, FVM_EFLUX_MINB)
     k_eflux(ArenaPtrs<R> A, int stage, int routine, int items) {
   static_assert(sizeof(R) == 8, "the FP64 pass");
+  __shared__ double s_face[8 * kEdgeThreads];
   int w0, nwork;
   work_range(A, w0, nwork);
   for (int i = w0 * items + blockIdx.x; i < nwork * items; i += gridDim.x) {
@@ -1205,17 +1244,20 @@ __global__ void __launch_bounds__(kEdgeThreads, 4)
     const MeshConst &mc = A.mc[bi.mesh];
     const R4<R> *P = A.st[cur_buf(ctl.phase, stage)];
     if (c == items - 1) {
-      for (int k = threadIdx.x; k < bi.nb; k += kEdgeThreads) {
-        const int b = bi.b0 + k;
-        boundary_flux<R>(A, mc, ctl, A.bb_nodes[b], P, A.bflux[2 * b], A.bflux[2 * b + 1]);
-      }
+      for (int k = threadIdx.x; k < 4 * bi.nb; k += kEdgeThreads)
+        boundary_row(A, mc, ctl, bi.b0 + k / 4, P, k & 3);
       continue;
     }
     const int k = c * kEdgeThreads + threadIdx.x;
     if (k >= A.blk_neo[bi.part]) continue;
     int err = 0;
+    R f[4];
+    edge_flux_f64<FLUX>(A, flux_const<R>(mc), P, bi.e0 + k, s_face + threadIdx.x, f, err);
     R4<R> o;
-    edge_flux_f64<FLUX>(A, flux_const<F64>(mc), P, bi.e0 + k, o, err);
+    o.x = f[0];
+    o.y = f[1];
+    o.z = f[2];
+    o.w = f[3];
     A.eflux[bi.e0 + k] = o;
     if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
   }
@@ -1605,7 +1647,7 @@ __global__ void __launch_bounds__(kBlockVerts) k_sa(ArenaPtrs<R> A, int stage, i
         }
       } else {
         const double2 c1 = A.coord[t.x], c2 = A.coord[t.y], c3 = A.coord[t.z];
-        areat = R(0.25 / A.elarea[t.w]);
+        areat = A.areat[t.w];
         dbxx[0] = R(c2.y - c3.y);
         dbxx[1] = R(c3.y - c1.y);
         dbxx[2] = R(c1.y - c2.y);

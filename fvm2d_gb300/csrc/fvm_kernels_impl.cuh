@@ -2,10 +2,34 @@
 // Included once per precision translation unit.
 #pragma once
 
+#include <cstring>
+
 #include "fvm_kernels.cuh"
 #include "fvm_launch.h"
 
 namespace fvm {
+
+// The arithmetic type of the kernels: F64 for FP64 states (products, quotients
+// and roots on the integer pipes, the same bits), float for FP32.  The fused
+// pass (off by default) keeps the hardware operations: it compiles for double.
+template <typename R>
+struct KernelType {
+  using T = R;
+};
+template <>
+struct KernelType<double> {
+  using T = F64;
+};
+template <typename R>
+using KT = typename KernelType<R>::T;
+template <typename R>
+inline ArenaPtrs<KT<R>> kptrs(const ArenaPtrs<R> &A) {
+  static_assert(sizeof(ArenaPtrs<KT<R>>) == sizeof(ArenaPtrs<R>) && sizeof(KT<R>) == sizeof(R),
+                "same arrays");
+  ArenaPtrs<KT<R>> o;
+  std::memcpy(&o, &A, sizeof(o));
+  return o;
+}
 
 // Grid of a persistent per-block kernel: one wave of the CTAs that fit on
 // the device at once (its occupancy with this shared memory), so that no
@@ -29,16 +53,16 @@ inline void launch_flux_code(const ArenaPtrs<R> &A, const LaunchCfg &c, int stag
                              int irk, int routine) {
   if constexpr (sizeof(R) == 4) {
     const size_t sm = size_t(c.max_slots) * sizeof(R4<R>);
-    k_flux<R, F><<<fit_grid(c, k_flux<R, F>, sm, kFluxThreads), kFluxThreads, sm, c.stream>>>(
-        A, stage, mode, irk, routine);
+    k_flux<KT<R>, F><<<fit_grid(c, k_flux<KT<R>, F>, sm, kFluxThreads), kFluxThreads, sm, c.stream>>>(
+        kptrs(A), stage, mode, irk, routine);
   } else {
     // a block's owned entries in items of kEdgeThreads, and its boundary edges
     const int items = (c.max_slots + kEdgeThreads - 1) / kEdgeThreads + 1;
     LaunchCfg ce = c;
     ce.grid = c.grid > INT_MAX / items ? INT_MAX : c.grid * items;
-    k_eflux<R, F><<<fit_grid(ce, k_eflux<R, F>, 0, kEdgeThreads), kEdgeThreads, 0, c.stream>>>(
-        A, stage, routine, items);
-    k_egather<R><<<fit_grid(c, k_egather<R>, 0), kBlockVerts, 0, c.stream>>>(A, stage, mode, irk,
+    k_eflux<KT<R>, F><<<fit_grid(ce, k_eflux<KT<R>, F>, 0, kEdgeThreads), kEdgeThreads, 0, c.stream>>>(
+        kptrs(A), stage, routine, items);
+    k_egather<KT<R>><<<fit_grid(c, k_egather<KT<R>>, 0), kBlockVerts, 0, c.stream>>>(kptrs(A), stage, mode, irk,
                                                                              routine);
   }
 }
@@ -68,14 +92,14 @@ template <typename R>
 inline cudaError_t flux_attributes(size_t f) {
   if constexpr (sizeof(R) == 4) {
     const int b = (int)f;
-    cudaError_t e = cudaFuncSetAttribute(k_flux<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 1 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 2 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<R, 3 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    cudaError_t e = cudaFuncSetAttribute(k_flux<KT<R>, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 1 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 2 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 3 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     return e;
   } else {
     return cudaSuccess;
@@ -92,7 +116,7 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_visc(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int do_dt,  \
                           int routine) {                                                   \
-    k_visc<R><<<fit_grid(c, k_visc<R>, 0), kBlockVerts, 0, c.stream>>>(A, stage, do_dt, routine);             \
+    k_visc<KT<R>><<<fit_grid(c, k_visc<KT<R>>, 0), kBlockVerts, 0, c.stream>>>(kptrs(A), stage, do_dt, routine);             \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_grad_pipe(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage,       \
@@ -106,12 +130,12 @@ inline cudaError_t flux_attributes(size_t f) {
     const size_t sb = (size_t)ns * pl.stage;                                               \
     const int vis = c.viscous ? 1 : 0;                                                     \
     if (groups == 1)                                                                       \
-      k_grad_pipe<R, 1><<<fit_grid(c, k_grad_pipe<R, 1>, sb, 32 + kBlockVerts),            \
-                          32 + kBlockVerts, sb, c.stream>>>(A, stage, do_dt, routine,      \
+      k_grad_pipe<KT<R>, 1><<<fit_grid(c, k_grad_pipe<KT<R>, 1>, sb, 32 + kBlockVerts),            \
+                          32 + kBlockVerts, sb, c.stream>>>(kptrs(A), stage, do_dt, routine,      \
                           c.max_tri, c.max_halo, vis, ns, budget, inject, skip_inviscid);  \
     else                                                                                   \
-      k_grad_pipe<R, 2><<<fit_grid(c, k_grad_pipe<R, 2>, sb, 32 + 2 * kBlockVerts),        \
-                          32 + 2 * kBlockVerts, sb, c.stream>>>(A, stage, do_dt, routine,  \
+      k_grad_pipe<KT<R>, 2><<<fit_grid(c, k_grad_pipe<KT<R>, 2>, sb, 32 + 2 * kBlockVerts),        \
+                          32 + 2 * kBlockVerts, sb, c.stream>>>(kptrs(A), stage, do_dt, routine,  \
                           c.max_tri, c.max_halo, vis, ns, budget, inject, skip_inviscid);  \
     return cudaGetLastError();                                                             \
   }                                                                                        \
@@ -124,8 +148,8 @@ inline cudaError_t flux_attributes(size_t f) {
     int skip = 0;                                                                          \
     if (sizeof(R) == 4 && c.stencil) {                                                     \
       if (c.any_inviscid) {                                                                \
-        k_grad_stencil<R><<<fit_grid(c, k_grad_stencil<R>, 0), kBlockVerts, 0, c.stream>>>( \
-            A, stage, do_dt, routine);                                                     \
+        k_grad_stencil<KT<R>><<<fit_grid(c, k_grad_stencil<KT<R>>, 0), kBlockVerts, 0, c.stream>>>( \
+            kptrs(A), stage, do_dt, routine);                                                     \
         const cudaError_t se = cudaGetLastError();                                         \
         if (se != cudaSuccess) return se;                                                  \
       }                                                                                    \
@@ -138,18 +162,18 @@ inline cudaError_t flux_attributes(size_t f) {
       if (pe != cudaErrorNotSupported) return pe;                                          \
     }                                                                                      \
     if (c.grad_mode == 2) {                                                                \
-      k_grad_v<R><<<fit_grid(c, k_grad_v<R>, 0), kBlockVerts, 0, c.stream>>>(A, stage, do_dt, routine, skip); \
+      k_grad_v<KT<R>><<<fit_grid(c, k_grad_v<KT<R>>, 0), kBlockVerts, 0, c.stream>>>(kptrs(A), stage, do_dt, routine, skip); \
       return cudaGetLastError();                                                           \
     }                                                                                      \
     if (c.grad_mode >= 3 && c.tri_loc) {  /* else the per-thread form, same sums */      \
       if (sizeof(R) != 4) return cudaErrorNotSupported;                                    \
       const size_t sb = grad_bulk_layout(c.max_tri, c.max_halo, c.viscous).total;          \
       if (sb > kMaxSmem) return cudaErrorInvalidConfiguration;                            \
-      k_grad_bulk<R><<<fit_grid(c, k_grad_bulk<R>, sb), kBlockVerts, sb, c.stream>>>(       \
-          A, stage, do_dt, routine, c.max_tri, c.max_halo, c.viscous ? 1 : 0, skip);       \
+      k_grad_bulk<KT<R>><<<fit_grid(c, k_grad_bulk<KT<R>>, sb), kBlockVerts, sb, c.stream>>>(       \
+          kptrs(A), stage, do_dt, routine, c.max_tri, c.max_halo, c.viscous ? 1 : 0, skip);       \
       return cudaGetLastError();                                                           \
     }                                                                                      \
-    k_grad<R><<<fit_grid(c, k_grad<R>, sm), kBlockVerts, sm, c.stream>>>(A, stage, do_dt, routine, c.max_tri, skip);  \
+    k_grad<KT<R>><<<fit_grid(c, k_grad<KT<R>>, sm), kBlockVerts, sm, c.stream>>>(kptrs(A), stage, do_dt, routine, c.max_tri, skip);  \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_flux(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,   \
@@ -180,47 +204,47 @@ inline cudaError_t flux_attributes(size_t f) {
   cudaError_t launch_sa(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int routine) {\
     size_t sm = smem_sa(c, (R *)nullptr);                                                  \
     if (sm > kMaxSmem) return cudaErrorInvalidConfiguration;                              \
-    k_sa<R><<<fit_grid(c, k_sa<R>, sm), kBlockVerts, sm, c.stream>>>(A, stage, routine, c.max_tri);           \
+    k_sa<KT<R>><<<fit_grid(c, k_sa<KT<R>>, sm), kBlockVerts, sm, c.stream>>>(kptrs(A), stage, routine, c.max_tri);           \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c) {                   \
     if (A.nslots <= 0) return cudaSuccess;                                                 \
-    k_monitor<R><<<A.nslots, monitor_threads<R>(), 0, c.stream>>>(A);                      \
+    k_monitor<KT<R>><<<A.nslots, monitor_threads<R>(), 0, c.stream>>>(kptrs(A));                      \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_update(const ArenaPtrs<R> &A, const LaunchCfg &c, int irk) {           \
-    k_update<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A, irk);                             \
+    k_update<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A), irk);                             \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_time_step(const ArenaPtrs<R> &A, const LaunchCfg &c) {                 \
-    k_time_step<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                               \
+    k_time_step<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                               \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_positivity(const ArenaPtrs<R> &A, const LaunchCfg &c) {                \
-    k_positivity<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                              \
+    k_positivity<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                              \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_conres(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int first) {\
-    k_conres_part<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                             \
-    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 0, first);                       \
+    k_conres_part<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                             \
+    k_routine_monitor<KT<R>><<<1, 256, 0, c.stream>>>(kptrs(A), mesh, 0, first);                       \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh) {             \
-    k_routine_monitor<R><<<1, 256, 0, c.stream>>>(A, mesh, 1, 0);                           \
+    k_routine_monitor<KT<R>><<<1, 256, 0, c.stream>>>(kptrs(A), mesh, 1, 0);                           \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_gradient_edge(const ArenaPtrs<R> &A, const LaunchCfg &c) {             \
     const size_t sm = size_t(c.max_slots) * sizeof(Grad<R>);                                 \
     if (sm > kMaxSmem) return cudaErrorInvalidConfiguration;                              \
-    k_gradient_edge<R><<<c.grid, kBlockVerts, sm, c.stream>>>(A);                          \
+    k_gradient_edge<KT<R>><<<c.grid, kBlockVerts, sm, c.stream>>>(kptrs(A));                          \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_shockind(const ArenaPtrs<R> &A, const LaunchCfg &c) {                  \
-    k_shockind<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                                \
+    k_shockind<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                                \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_limitgrad(const ArenaPtrs<R> &A, const LaunchCfg &c) {                 \
-    k_limitgrad<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                               \
+    k_limitgrad<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                               \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t prepare_attributes(const LaunchCfg &c, R *) {                                \
@@ -237,22 +261,22 @@ inline cudaError_t flux_attributes(size_t f) {
       if (k == 3) e2 = cudaFuncSetAttribute(k_step<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
       if (e2 != cudaSuccess) return e2;                                                    \
     }                                                                                      \
-    cudaError_t e = cudaFuncSetAttribute(k_grad<R>,                                        \
+    cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>>,                                        \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g); \
     if (e == cudaSuccess) e = flux_attributes<R>(f);                                       \
     if (e == cudaSuccess)                                                                  \
-      e = cudaFuncSetAttribute(k_sa<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s); \
+      e = cudaFuncSetAttribute(k_sa<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s); \
     const size_t gb = grad_bulk_layout(c.max_tri, kTriLocMax, c.viscous).total;            \
     if (e == cudaSuccess && sizeof(R) == 4 && gb <= kMaxSmem)                              \
-      e = cudaFuncSetAttribute(k_grad_bulk<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gb); \
+      e = cudaFuncSetAttribute(k_grad_bulk<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gb); \
     const size_t ge = size_t(c.max_slots) * sizeof(Grad<R>);                                 \
     if (e == cudaSuccess && ge <= kMaxSmem)                                                \
-      e = cudaFuncSetAttribute(k_gradient_edge<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ge); \
+      e = cudaFuncSetAttribute(k_gradient_edge<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ge); \
     const int pmax = (int)(kMaxSmem - kPipeStaticSmem);                                    \
     if (e == cudaSuccess && sizeof(R) == 4)                                                \
-      e = cudaFuncSetAttribute(k_grad_pipe<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
+      e = cudaFuncSetAttribute(k_grad_pipe<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
     if (e == cudaSuccess && sizeof(R) == 4)                                                \
-      e = cudaFuncSetAttribute(k_grad_pipe<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
+      e = cudaFuncSetAttribute(k_grad_pipe<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
     return e;                                                                              \
   }
 

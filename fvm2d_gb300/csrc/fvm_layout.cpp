@@ -457,7 +457,7 @@ int64_t verify_layout(const MeshLayout &L) {
     // the bulk-copy gradient pass stages [vt0, vt0 + nvt) in a tile of
     // 3 * max_tri + 16 entries and the block's vertex ranges from v0
     if (bi.vt0 != L.vt_ptr[bi.v0] || bi.nvt != L.vt_ptr[bi.v0 + bi.nv] - bi.vt0 ||
-        bi.nvt > 3 * bi.nt || bi.v0 % kBlockVerts != 0)
+        bi.nvt > 3 * bi.nt || bi.v0 % kVertAlign != 0)
       bad++;
     // own vertices: triangles among the block's own, ascending
     for (int v = bi.v0; v < bi.v0 + bi.nv; v++) {
