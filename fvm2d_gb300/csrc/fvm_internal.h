@@ -143,7 +143,7 @@ struct MeshConst {
   int blk0, nblk;                   // range in the block table
   int sw0, nsw;                     // solid edges (sw_nodes)
   int orig123[3];                   // arena ids of driver vertices 1,2,3
-  int pad0;
+  int sub;                          // blocks a leaf of kBlockVerts vertices is split into (1, 2, 4)
   double gamma, gamma1, gas_const, pi, prandtl, prandtl_turb;
   double albada11, albada12, albada21, albada22, epsilon;
   double cb1, cb2, sigma_sa, kolm, cw1, cw2, cw3, cv1, cv2;

@@ -761,6 +761,14 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRADV_MINB32
 // slow, and this keeps it out of the reduction: the sum carries ~2^-47
 // relative error instead of 2^-53; max |gra| is exact.
 // ---------------------------------------------------------------------------
+// The sums of a block's eight warps (32 consecutive vertices each) are added
+// in pairs, and a mesh whose leaves of 256 vertices are split into smaller
+// blocks adds those blocks' records in the same pairs (conres_block), so the
+// norm does not depend on the split.
+static_assert(kBlockVerts == 256, "eight warps");
+__device__ __forceinline__ double warp_sums(const double *s) {
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
 struct DFloat {
   float hi, lo;
 };
@@ -846,10 +854,11 @@ __device__ __forceinline__ void block_conres_partial(bool have, R rho_new, R rho
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      DFloat t = s_sq[0], m = s_mx[0];
+      const DFloat t = df_add(df_add(df_add(s_sq[0], s_sq[1]), df_add(s_sq[2], s_sq[3])),
+                              df_add(df_add(s_sq[4], s_sq[5]), df_add(s_sq[6], s_sq[7])));
+      DFloat m = s_mx[0];
       int a = s_arg[0];
-      for (int i = 1; i < (int)(blockDim.x >> 5); i++) {
-        t = df_add(t, s_sq[i]);
+      for (int i = 1; i < kBlockVerts / 32; i++) {
         if (df_greater(s_mx[i], m) || (s_mx[i].hi == m.hi && s_mx[i].lo == m.lo && s_arg[i] < a)) {
           m = s_mx[i];
           a = s_arg[i];
@@ -866,17 +875,16 @@ __device__ __forceinline__ void block_conres_partial(bool have, R rho_new, R rho
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double sacc = 0.0, m = 0.0;
+    double m = 0.0;
     int a = INT_MAX;
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
-      sacc += s_red[i];
+    for (int i = 0; i < kBlockVerts / 32; i++) {
       if (s_max[i] > m || (s_max[i] == m && s_arg[i] < a)) {
         m = s_max[i];
         a = s_arg[i];
       }
     }
     BlockPartial bp;
-    bp.sumsq = sacc;
+    bp.sumsq = warp_sums(s_red);
     bp.maxabs = m;
     bp.argmax = a;
     bp.pad = 0;
@@ -1923,25 +1931,35 @@ __device__ void conres_block(const ArenaPtrs<R> &A, const MeshConst &mc, double 
   double s = 0.0, m = 0.0;
   int a = INT_MAX;
   // the mesh's partials are contiguous (block k's record is blk0 + k);
-  // eight loads in flight per thread (a 2048-block mesh in one trip),
-  // folded in index order
+  // eight loads in flight per thread (a 2048-block mesh in one trip): the
+  // records of 8 / sub leaves, each leaf's `sub` records added in pairs and
+  // the leaves in order
   constexpr int kU = 8;
-  for (int i0 = threadIdx.x; i0 < mc.nblk; i0 += kU * blockDim.x) {
+  const int sub = mc.sub, nleaf = (mc.nblk + sub - 1) / sub;
+  for (int i0 = threadIdx.x; i0 < nleaf; i0 += kU / sub * blockDim.x) {
     BlockPartial bp[kU];
 #pragma unroll
     for (int u = 0; u < kU; u++) {
-      const int i = i0 + u * (int)blockDim.x;
-      if (i < mc.nblk) bp[u] = A.part[mc.blk0 + i];
+      const int i = (i0 + u / sub * (int)blockDim.x) * sub + u % sub;
+      if (i < mc.nblk && i0 + u / sub * (int)blockDim.x < nleaf) bp[u] = A.part[mc.blk0 + i];
+      else bp[u] = BlockPartial{0.0, 0.0, INT_MAX, 0};
+    }
+    if (sub == 4) {
+      s += (bp[0].sumsq + bp[1].sumsq) + (bp[2].sumsq + bp[3].sumsq);
+      s += (bp[4].sumsq + bp[5].sumsq) + (bp[6].sumsq + bp[7].sumsq);
+    } else if (sub == 2) {
+#pragma unroll
+      for (int u = 0; u < kU; u += 2) s += bp[u].sumsq + bp[u + 1].sumsq;
+    } else {
+#pragma unroll
+      for (int u = 0; u < kU; u++) s += bp[u].sumsq;
     }
 #pragma unroll
-    for (int u = 0; u < kU; u++) {
-      if (i0 + u * (int)blockDim.x >= mc.nblk) break;
-      s += bp[u].sumsq;
+    for (int u = 0; u < kU; u++)
       if (bp[u].maxabs > m || (bp[u].maxabs == m && bp[u].argmax < a)) {
         m = bp[u].maxabs;
         a = bp[u].argmax;
       }
-    }
   }
   s_s[threadIdx.x] = s;
   s_m[threadIdx.x] = m;
@@ -2109,17 +2127,16 @@ __global__ void __launch_bounds__(kBlockVerts) k_conres_part(ArenaPtrs<R> A) {
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      double s = 0.0, m = 0.0;
+      double m = 0.0;
       int a = INT_MAX;
-      for (int i = 0; i < (int)(blockDim.x >> 5); i++) {
-        s += s_red[i];
+      for (int i = 0; i < kBlockVerts / 32; i++) {
         if (s_max[i] > m || (s_max[i] == m && s_arg[i] < a)) {
           m = s_max[i];
           a = s_arg[i];
         }
       }
       BlockPartial bp;
-      bp.sumsq = s;
+      bp.sumsq = warp_sums(s_red);
       bp.maxabs = m;
       bp.argmax = a;
       bp.pad = 0;

@@ -128,7 +128,18 @@ int32_t build_layout(const fvm_mesh &m, int bv, bool owned_first, MeshLayout &L)
     }
   }
   std::vector<int> block_start;
-  order_vertices(np, deg, adj, bv, L.perm, block_start);
+  order_vertices(np, deg, adj, kBlockVerts, L.perm, block_start);
+  // leaves split into blocks of bv consecutive vertices (the order, and so
+  // every sum over vertices, is that of whole leaves)
+  L.sub = kBlockVerts / bv;
+  if (L.sub > 1) {
+    std::vector<int> split;
+    for (size_t b = 0; b < block_start.size(); b++) {
+      const int end = b + 1 < block_start.size() ? block_start[b + 1] : np;
+      for (int v = block_start[b]; v < end; v += bv) split.push_back(v);
+    }
+    block_start.swap(split);
+  }
   L.iperm.assign(np, -1);
   for (int i = 0; i < np; i++) L.iperm[L.perm[i]] = i;
   const int nblk = (int)block_start.size();

@@ -16,6 +16,7 @@ namespace fvm {
 // the arena offsets.
 struct MeshLayout {
   int np = 0, nt = 0, nblk = 0;
+  int sub = 1;                    // blocks per leaf of kBlockVerts vertices
   std::vector<int> perm;          // new vertex -> driver vertex (0-based)
   std::vector<int> iperm;         // driver vertex -> new vertex
   std::vector<BlockInfo> blocks;  // v0,e0,b0,t0 relative; mesh/part filled at upload
@@ -44,7 +45,8 @@ struct MeshLayout {
   int max_halo = 0;               // max halo vertices of a block
 };
 
-// Builds the layout (owned_first: each block's own edges first in its list,
+// Builds the layout in blocks of block_verts vertices (kBlockVerts, or a half
+// or a quarter of it; owned_first: each block's own edges first in its list,
 // and ve_src, for FP64 batches); returns FVM_OK or FVM_ERR_ARG (bad connectivity) /
 // FVM_ERR_CAPACITY (a block needs more slots than the incidence entries can
 // address).
