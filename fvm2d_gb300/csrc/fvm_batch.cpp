@@ -2077,14 +2077,16 @@ extern "C" int32_t fvm_gpu_wall_dist(int32_t np, int32_t ne, const double *coord
   int2 *ds = nullptr;
   int *dp = nullptr;
   double *dw = nullptr;
+  unsigned char *scratch = nullptr;
   cudaError_t e = cudaSuccess;
-  if ((e = dalloc(O, &dc, np)) == cudaSuccess && (e = dalloc(O, &ds, sedge.size())) == cudaSuccess &&
+  if ((e = dalloc(O, &scratch, wall_scratch((int)sedge.size()))) == cudaSuccess &&
+      (e = dalloc(O, &dc, np)) == cudaSuccess && (e = dalloc(O, &ds, sedge.size())) == cudaSuccess &&
       (e = dalloc(O, &dp, np)) == cudaSuccess && (e = dalloc(O, &dw, np)) == cudaSuccess &&
       (e = cudaMemcpy(dc, coord, 16 * (size_t)np, cudaMemcpyHostToDevice)) == cudaSuccess &&
       (sedge.empty() ||
        (e = cudaMemcpy(ds, sedge.data(), 8 * sedge.size(), cudaMemcpyHostToDevice)) == cudaSuccess) &&
       (e = cudaMemcpy(dp, ptype, 4 * (size_t)np, cudaMemcpyHostToDevice)) == cudaSuccess &&
-      (e = launch_wall_dist(np, (int)sedge.size(), dc, ds, dp, bugcompat, dw, 0)) == cudaSuccess)
+      (e = launch_wall_dist(np, (int)sedge.size(), dc, ds, dp, bugcompat, dw, scratch, 0)) == cudaSuccess)
     e = cudaMemcpy(wd, dw, 8 * (size_t)np, cudaMemcpyDeviceToHost);
   for (void *p : O) cudaFree(p);
   return cuda_status(nullptr, e);

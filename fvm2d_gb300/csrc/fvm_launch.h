@@ -77,7 +77,9 @@ cudaError_t launch_edge_csl(const double2 *ds, D4 *csl, int n, cudaStream_t s);
 cudaError_t launch_dtlength(int np, int nt, const double2 *coord, const int *elem,
                             const double *elarea, double *drmin, cudaStream_t s);
 cudaError_t launch_wall_dist(int np, int nsedge, const double2 *coord, const int2 *sedge,
-                             const int *ptype, int bugcompat, double *wd, cudaStream_t s);
+                             const int *ptype, int bugcompat, double *wd, void *scratch,
+                             cudaStream_t s);
+size_t wall_scratch(int nsedge);   // bytes of its scratch
 // driver-order FP64 <-> arena-order per-vertex arrays of one mesh (fvm_setup.cu)
 cudaError_t launch_get_vertex(int rsz, double *dst, const unsigned char *src, size_t stride,
                               const int *orig, int np, int k, int c0, cudaStream_t s);
