@@ -134,6 +134,7 @@ struct fvm_batch {
   BlockInfo *blocks = nullptr;
   BlockInfo *wblocks = nullptr;   // blocks[work[w]], refreshed with the work list
   int2 *be_nodes = nullptr, *sw_nodes = nullptr;
+  float2 *sw_vec = nullptr;   // FP32
   double2 *be_ds = nullptr;
   D4 *be_csl = nullptr;
   int4 *bb_nodes = nullptr, *bt_nodes = nullptr;
@@ -252,6 +253,7 @@ ArenaPtrs<R> ptrs(const fvm_batch *b) {
   A.hl_ptr = b->hl_ptr;
   A.hl_list = b->hl_list;
   A.sw_nodes = b->sw_nodes;
+  A.sw_vec = b->sw_vec;
   A.va_rng = b->va_rng;
   A.va_list = b->va_list;
   A.va_w = b->va_w;
@@ -844,6 +846,7 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
     TRYB(dalloc(O, &b->drmin32, V));
     TRYB(dalloc(O, &b->wd32, V));
     TRYB(dalloc(O, &b->tri_g32, (size_t)c.tri_entries));
+    TRYB(dalloc(O, &b->sw_vec, (size_t)c.solid_edges));
   }
   TRYB(dalloc(O, &b->sw_nodes, (size_t)c.solid_edges));
   TRYB(dalloc(O, &b->mc, (size_t)c.meshes));
@@ -1095,7 +1098,7 @@ extern "C" int64_t fvm_prepared_bytes(const fvm_prepared *prep, int32_t precisio
   bytes += (int64_t)L.be_nodes.size() * (8 + 16 + (r == 4 ? 16 : 64));
   bytes += (int64_t)L.bb_nodes.size() * (r == 4 ? 16 : 80) + (int64_t)L.bt_nodes.size() * (16 + (r == 4 ? 32 : 0));
   bytes += (int64_t)L.nt * 8 + (int64_t)L.ve_list.size() * (r == 4 ? 2 : 6) + (int64_t)L.vt_list.size() * 2;
-  bytes += (int64_t)L.va_list.size() * (12 + (r == 4 ? 8 : 0)) + (int64_t)L.sw_nodes.size() * 8;
+  bytes += (int64_t)L.va_list.size() * (12 + (r == 4 ? 8 : 0)) + (int64_t)L.sw_nodes.size() * (r == 4 ? 16 : 8);
   bytes += (int64_t)L.nblk * (sizeof(BlockInfo) + sizeof(BlockPartial) + 4);
   bytes += (int64_t)L.be_loc.size() * 4 + (int64_t)L.halo_ids.size() * 4;
   bytes += (int64_t)L.hl_ptr.size() * 4 + (int64_t)L.hl_list.size() * 2;
@@ -1269,6 +1272,15 @@ static int32_t add_prepared(fvm_batch *b, fvm_prepared *prep, int32_t *slot_out,
   if (b->va_w) PUT(put_range(b, b->va_w, S.off[P_VA], prep->va_w, us));
   PUT(put_range(b, b->va_dsl, S.off[P_VA], prep->va_dsl, us));
   PUT(put_range(b, b->sw_nodes, S.off[P_SW], sw, us));
+  std::vector<float2> swv;
+  if (b->sw_vec) {
+    swv.resize(L.sw_nodes.size());
+    for (size_t i = 0; i < swv.size(); i++) {
+      const double2 c1 = prep->coord[L.sw_nodes[i].x], c2 = prep->coord[L.sw_nodes[i].y];
+      swv[i] = make_float2((float)(c2.y - c1.y), -(float)(c2.x - c1.x));
+    }
+    PUT(put_range(b, b->sw_vec, S.off[P_SW], swv, us));
+  }
   PUT(cudaMemcpyAsync(b->mc + sid, &mc, sizeof(mc), cudaMemcpyHostToDevice, us));
   PUT(cudaMemcpyAsync(b->ctl + sid, &ctl, sizeof(ctl), cudaMemcpyHostToDevice, us));
   const size_t r = b->rsz;

@@ -256,6 +256,7 @@ struct ArenaPtrs {
   const TriGeo32 *tri_g32; // FP32 path: per triangle entry of the blocks (bt_* order)
   // solid edges per mesh for clcd (n1, n2) in beindx order
   const int2 *sw_nodes;
+  const float2 *sw_vec;   // FP32: y(n2)-y(n1), x(n1)-x(n2) of each, FP64 differences rounded once
   // fused gradient+flux pass: local slots of edge ends, halo vertices and
   // their triangle incidence (slot | pos << 14 in the block's bt list)
   const uint32_t *be_loc;

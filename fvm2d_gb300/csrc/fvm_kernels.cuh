@@ -167,11 +167,9 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Threads of the per-mesh monitor CTA (a power of two; the fixed-order
-// reduction trees depend on it).  Wider CTAs measured no faster.
+// Threads of the per-mesh monitor CTA (eight warps; the fixed-order reduction
+// depends on it).  Wider CTAs measured no faster.
 constexpr int kMonitorMaxThreads = 256;
-template <typename R>
-constexpr int monitor_threads() { return 256; }
 
 // Per-vertex geometry in the kernel's precision (FP32 copies for R = float).
 template <typename R>
@@ -1767,12 +1765,12 @@ __global__ void __launch_bounds__(kBlockVerts) k_sa(ArenaPtrs<R> A, int stage, i
 // the serial Fortran chain.
 // ---------------------------------------------------------------------------
 // FP32 states: one solid edge's pressure and viscous force (clcd.f:20-40),
-// the terms from the FP32 values (the edge vector an FP64 difference rounded
-// once), accumulated in FP64.
-__device__ __forceinline__ void wall_force(double2 c1, double2 c2, float mu1, float mu2,
+// the terms from the FP32 values (sv: the edge's normal, FP64 differences
+// rounded once), accumulated in FP64.
+__device__ __forceinline__ void wall_force(float2 sv, float mu1, float mu2,
                                            const Grad<float> &g1, const Grad<float> &g2, float p1,
                                            float p2, double &xf, double &yf) {
-  const float sx = float(c2.y - c1.y), sy = -float(c2.x - c1.x);
+  const float sx = sv.x, sy = sv.y;
   const float n2b3 = 2.0f / 3.0f;
   const float txx = 0.5f * (n2b3 * mu1 * (2.0f * g1.qx[1] - g1.qy[2]) +
                             n2b3 * mu2 * (2.0f * g2.qx[1] - g2.qy[2]));
@@ -1787,8 +1785,8 @@ __device__ __forceinline__ void wall_force(double2 c1, double2 c2, float mu1, fl
 // FP64, the Fortran chain: clcd.f:34-40 adds three terms per solid edge, one
 // after another, so the additions are serial; nothing else is.  All threads
 // form the terms of a tile of edges in shared memory, then one thread per
-// component adds them in edge order while the other warps form the next
-// tile.  Each addition costs one pass through the FP64 pipe (about 32 ns on
+// component adds them in edge order while the other warps sum the residual
+// and form the next tile.  Each addition costs one pass through the FP64 pipe (about 32 ns on
 // this GPU, 2 lanes per SM quarter-cycle), which bounds the chain: with the
 // loads and products of every edge inside it the chain took 1.45 ms for 1024
 // edges, k_monitor 1480 us against FORCE_US us now.  mu = 0 (inviscid meshes)
@@ -1843,146 +1841,185 @@ __device__ __forceinline__ double force_chain(const ForceTile &s, int comp, int 
   return v;
 }
 
-template <typename R>
-__device__ void clcd_block(const ArenaPtrs<R> &A, const MeshConst &mc, int mesh_phase,
-                           double &cl, double &cd) {
-  const R4<R> *P = A.st[mesh_phase];
-  double xf = 0.0, yf = 0.0;
-  if constexpr (sizeof(R) == 8) {
-    __shared__ ForceTile s_f[2];
-    __shared__ double s_v[2];
-    // warp 0 (lanes 0 and 1) adds tile i while the others form tile i + 1
-    const int nt = (mc.nsw + kForceTile - 1) / kForceTile;
-    double v = 0.0;
-    bool some = false;   // of the tile formed last
-    for (int k = threadIdx.x; k < min(mc.nsw, kForceTile); k += blockDim.x)
-      some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + k], k, s_f[0]);
-    for (int i = 0; i < nt; i++) {
-      const bool viscous = __syncthreads_or(some);
-      some = false;
-      if (threadIdx.x < 32) {
-        if (threadIdx.x < 2)
-          v = force_chain(s_f[i & 1], threadIdx.x, min(mc.nsw - i * kForceTile, kForceTile),
-                          viscous, v);
-      } else if (i + 1 < nt) {
-        const int base = (i + 1) * kForceTile, n = min(mc.nsw - base, kForceTile);
-        for (int k = threadIdx.x - 32; k < n; k += blockDim.x - 32)
-          some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + base + k], k, s_f[(i + 1) & 1]);
-      }
-    }
-    if (threadIdx.x < 2) s_v[threadIdx.x] = v;
-    __syncthreads();
-    xf = s_v[0];
-    yf = s_v[1];
-  } else {
-    // each thread's edges i, i + blockDim, ... summed in that order, with
-    // the loads of four edges issued together per trip
-    __shared__ double s_x[kMonitorMaxThreads], s_y[kMonitorMaxThreads];
-    constexpr int kU = 4;
-    const int nt = (int)blockDim.x;
-    for (int i0 = threadIdx.x; i0 < mc.nsw; i0 += kU * nt) {
-      int2 nn[kU];
-#pragma unroll
-      for (int u = 0; u < kU; u++)
-        nn[u] = (i0 + u * nt < mc.nsw) ? A.sw_nodes[mc.sw0 + i0 + u * nt] : make_int2(0, 0);
-      double2 c1[kU], c2[kU];
-      R mu1[kU], mu2[kU], p1[kU], p2[kU];
-      Grad<R> g1[kU], g2[kU];
-#pragma unroll
-      for (int u = 0; u < kU; u++) {
-        c1[u] = A.coord[nn[u].x];
-        c2[u] = A.coord[nn[u].y];
-        mu1[u] = A.mu[nn[u].x];
-        mu2[u] = A.mu[nn[u].y];
-        g1[u] = A.grad[nn[u].x];
-        g2[u] = A.grad[nn[u].y];
-        p1[u] = P[nn[u].x].w;
-        p2[u] = P[nn[u].y].w;
-      }
-#pragma unroll
-      for (int u = 0; u < kU; u++) {
-        if (i0 + u * nt >= mc.nsw) break;
-        wall_force(c1[u], c2[u], mu1[u], mu2[u], g1[u], g2[u], p1[u], p2[u], xf, yf);
-      }
-    }
-    s_x[threadIdx.x] = xf;
-    s_y[threadIdx.x] = yf;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) {
-        s_x[threadIdx.x] += s_x[threadIdx.x + s];
-        s_y[threadIdx.x] += s_y[threadIdx.x + s];
-      }
-      __syncthreads();
-    }
-    xf = s_x[0];
-    yf = s_y[0];
+// What the monitor reduces over a mesh: the sum of gra^2 and the largest |gra|
+// with its first driver index (conres.f:14-22), and the force on the wall.
+struct Moments {
+  double s, x, y, m;
+  int a;
+};
+
+// (m, a) with a larger maximum or, at the same one, a smaller index; m >= 0 and
+// never NaN, so the bits order like the values (no FP64 comparison)
+__device__ __forceinline__ void max_first(double &m, int &a, double om, int oa) {
+  const long long x = __double_as_longlong(m), y = __double_as_longlong(om);
+  if (y > x || (y == x && oa < a)) {
+    m = om;
+    a = oa;
   }
-  const double q = 0.5 * mc.r_inf * (mc.q_inf * mc.q_inf);
-  cl = (-mc.sin_aoa * xf + mc.cos_aoa * yf) / q;
-  cd = (mc.cos_aoa * xf + mc.sin_aoa * yf) / q;
+}
+template <int N>
+__device__ __forceinline__ void reduce_residual(Moments &v) {
+#pragma unroll
+  for (int off = N / 2; off > 0; off >>= 1) {
+    v.s += __shfl_xor_sync(0xffffffffu, v.s, off);
+    max_first(v.m, v.a, __shfl_xor_sync(0xffffffffu, v.m, off),
+              __shfl_xor_sync(0xffffffffu, v.a, off));
+  }
+}
+template <int N>
+__device__ __forceinline__ void reduce_force(Moments &v) {
+#pragma unroll
+  for (int off = N / 2; off > 0; off >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+  }
 }
 
+// A thread's share of a mesh's conres partials: thread t of n.  The partials
+// are contiguous (block k's record is blk0 + k); eight loads in flight per
+// thread (a 2048-block mesh in one trip): the records of 8 / sub leaves, each
+// leaf's `sub` records added in pairs and the leaves in order.
 template <typename R>
-__device__ void conres_block(const ArenaPtrs<R> &A, const MeshConst &mc, double &sum,
-                             double &mx, int &arg) {
-  __shared__ double s_s[kMonitorMaxThreads], s_m[kMonitorMaxThreads];
-  __shared__ int s_a[kMonitorMaxThreads];
-  double s = 0.0, m = 0.0;
-  int a = INT_MAX;
-  // the mesh's partials are contiguous (block k's record is blk0 + k);
-  // eight loads in flight per thread (a 2048-block mesh in one trip): the
-  // records of 8 / sub leaves, each leaf's `sub` records added in pairs and
-  // the leaves in order
+__device__ __forceinline__ void conres_share(const ArenaPtrs<R> &A, const MeshConst &mc, int t,
+                                             int n, Moments &v) {
   constexpr int kU = 8;
   const int sub = mc.sub, nleaf = (mc.nblk + sub - 1) / sub;
-  for (int i0 = threadIdx.x; i0 < nleaf; i0 += kU / sub * blockDim.x) {
+  for (int i0 = t; i0 < nleaf; i0 += kU / sub * n) {
     BlockPartial bp[kU];
 #pragma unroll
     for (int u = 0; u < kU; u++) {
-      const int i = (i0 + u / sub * (int)blockDim.x) * sub + u % sub;
-      if (i < mc.nblk && i0 + u / sub * (int)blockDim.x < nleaf) bp[u] = A.part[mc.blk0 + i];
+      const int leaf = i0 + u / sub * n, i = leaf * sub + u % sub;
+      if (leaf < nleaf && i < mc.nblk) bp[u] = A.part[mc.blk0 + i];
       else bp[u] = BlockPartial{0.0, 0.0, INT_MAX, 0};
     }
     if (sub == 4) {
-      s += (bp[0].sumsq + bp[1].sumsq) + (bp[2].sumsq + bp[3].sumsq);
-      s += (bp[4].sumsq + bp[5].sumsq) + (bp[6].sumsq + bp[7].sumsq);
+      v.s += (bp[0].sumsq + bp[1].sumsq) + (bp[2].sumsq + bp[3].sumsq);
+      if (i0 + n < nleaf) v.s += (bp[4].sumsq + bp[5].sumsq) + (bp[6].sumsq + bp[7].sumsq);
     } else if (sub == 2) {
 #pragma unroll
-      for (int u = 0; u < kU; u += 2) s += bp[u].sumsq + bp[u + 1].sumsq;
+      for (int u = 0; u < kU; u += 2)
+        if (i0 + u / 2 * n < nleaf) v.s += bp[u].sumsq + bp[u + 1].sumsq;
     } else {
 #pragma unroll
-      for (int u = 0; u < kU; u++) s += bp[u].sumsq;
+      for (int u = 0; u < kU; u++)
+        if (i0 + u * n < nleaf) v.s += bp[u].sumsq;
     }
 #pragma unroll
-    for (int u = 0; u < kU; u++)
-      if (bp[u].maxabs > m || (bp[u].maxabs == m && bp[u].argmax < a)) {
-        m = bp[u].maxabs;
-        a = bp[u].argmax;
-      }
+    for (int u = 0; u < kU; u++) max_first(v.m, v.a, bp[u].maxabs, bp[u].argmax);
   }
-  s_s[threadIdx.x] = s;
-  s_m[threadIdx.x] = m;
-  s_a[threadIdx.x] = a;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) {
-      s_s[threadIdx.x] += s_s[threadIdx.x + st];
-      const double om = s_m[threadIdx.x + st];
-      const int oa = s_a[threadIdx.x + st];
-      if (om > s_m[threadIdx.x] || (om == s_m[threadIdx.x] && oa < s_a[threadIdx.x])) {
-        s_m[threadIdx.x] = om;
-        s_a[threadIdx.x] = oa;
-      }
-    }
-    __syncthreads();
-  }
-  sum = s_s[0];
-  mx = s_m[0];
-  arg = s_a[0];
 }
 
-// One CTA (256 threads) per mesh slot listed in mesh_list.
+// FP32 states: a thread's share of the wall edges, i, i + n, ... summed in
+// that order, with the loads of four edges issued together per trip.
+__device__ __forceinline__ void force_share(const ArenaPtrs<float> &A, const MeshConst &mc,
+                                            const R4<float> *P, int t, int n, Moments &v) {
+  constexpr int kU = 4;
+  for (int i0 = t; i0 < mc.nsw; i0 += kU * n) {
+    int2 nn[kU];
+    float2 sv[kU];
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      const bool in = i0 + u * n < mc.nsw;
+      nn[u] = in ? A.sw_nodes[mc.sw0 + i0 + u * n] : make_int2(mc.v0, mc.v0);
+      sv[u] = in ? A.sw_vec[mc.sw0 + i0 + u * n] : make_float2(0.f, 0.f);
+    }
+    float mu1[kU], mu2[kU], p1[kU], p2[kU];
+    Grad<float> g1[kU], g2[kU];
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      mu1[u] = A.mu[nn[u].x];
+      mu2[u] = A.mu[nn[u].y];
+      g1[u] = A.grad[nn[u].x];
+      g2[u] = A.grad[nn[u].y];
+      p1[u] = P[nn[u].x].w;
+      p2[u] = P[nn[u].y].w;
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++) {
+      if (i0 + u * n >= mc.nsw) break;
+      wall_force(sv[u], mu1[u], mu2[u], g1[u], g2[u], p1[u], p2[u], v.x, v.y);
+    }
+  }
+}
+
+// The monitor's reduction, by all kMonitorMaxThreads threads (`what`: 1 the
+// residual, 2 the force, 3 both).  Warp 0 returns the residual's part and
+// warps 1 and 2 the force.  One CTA does this between two iterations, so its
+// latency counts and an FP64 operation of a warp costs 64 cycles: comparisons
+// read the bits, each reduction is five shuffles and one exchange, and the
+// final scalars are formed by different warps.  8 x 1024x384, alone, 22.4 us
+// as two 8-level shared-memory trees with one thread finishing; now 16.3 us (160 x 48: 9.6, now 5.2).
+template <typename R>
+__device__ __forceinline__ Moments mesh_moments(const ArenaPtrs<R> &A, const MeshConst &mc,
+                                                const R4<R> *P, int what) {
+  __shared__ Moments s_w[kMonitorMaxThreads / 32];
+  __shared__ double s_v[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Moments v = {0.0, 0.0, 0.0, 0.0, INT_MAX};
+  if constexpr (sizeof(R) == 4) {
+    if (what & 1) conres_share<R>(A, mc, threadIdx.x, kMonitorMaxThreads, v);
+    if (what & 2) {
+      force_share(A, mc, P, threadIdx.x, kMonitorMaxThreads, v);
+      reduce_force<32>(v);
+    }
+  } else {
+    // warp 0 (lanes 0 and 1) adds tile i while the others sum the residual and
+    // form tile i + 1
+    __shared__ ForceTile s_f[2];
+    const int nt = what & 2 ? (mc.nsw + kForceTile - 1) / kForceTile : 0;
+    double f = 0.0;
+    bool some = false;   // of the tile formed last
+    if (nt > 0)
+      for (int k = threadIdx.x; k < min(mc.nsw, kForceTile); k += kMonitorMaxThreads)
+        some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + k], k, s_f[0]);
+    for (int i = 0; i < nt || i == 0; i++) {
+      const bool viscous = __syncthreads_or(some);
+      some = false;
+      if (warp == 0) {
+        if (lane < 2 && i < nt)
+          f = force_chain(s_f[i & 1], lane, min(mc.nsw - i * kForceTile, kForceTile), viscous, f);
+      } else {
+        if (i == 0 && (what & 1))
+          conres_share<R>(A, mc, threadIdx.x - 32, kMonitorMaxThreads - 32, v);
+        if (i + 1 < nt) {
+          const int base = (i + 1) * kForceTile, n = min(mc.nsw - base, kForceTile);
+          for (int k = threadIdx.x - 32; k < n; k += kMonitorMaxThreads - 32)
+            some |= force_terms<R>(A, P, A.sw_nodes[mc.sw0 + base + k], k, s_f[(i + 1) & 1]);
+        }
+      }
+    }
+    if (threadIdx.x < 2) s_v[threadIdx.x] = f;
+  }
+  if (what & 1) reduce_residual<32>(v);
+  if (lane == 0) s_w[warp] = v;
+  __syncthreads();
+  if (warp > 2) return v;
+  v = s_w[lane & 7];
+  if (warp == 0) {
+    reduce_residual<8>(v);
+  } else if constexpr (sizeof(R) == 4) {
+    reduce_force<8>(v);
+  } else {
+    v.x = s_v[0];
+    v.y = s_v[1];
+  }
+  return v;
+}
+
+// clcd.f:43-46: the lift (k = 0) or drag coefficient from the wall force
+__device__ __forceinline__ double force_coefficient(const MeshConst &mc, const Moments &v, int k) {
+  const double q = 0.5 * mc.r_inf * (mc.q_inf * mc.q_inf);
+  return div64(k == 0 ? -mc.sin_aoa * v.x + mc.cos_aoa * v.y
+                      : mc.cos_aoa * v.x + mc.sin_aoa * v.y,
+               q);
+}
+// conres.f:23
+__device__ __forceinline__ double residual_norm(const MeshConst &mc, const Moments &v) {
+  return sqrt64(div64(v.s, double(mc.nv)));
+}
+
+// One CTA (256 threads) per mesh slot.  Thread 0 finishes the residual, the
+// verdict and the control block; threads 32 and 64 the lift and drag.
 template <typename R>
 __global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A) {
   const int m = blockIdx.x;
@@ -1990,30 +2027,37 @@ __global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A) 
   if (!ctl.active) return;
   if (A.wpart > 0 && A.mesh_part[m] != A.wpart) return;   // another chain's mesh
   const MeshConst &mc = A.mc[m];
-  double sum, mx;
-  int arg;
-  conres_block<R>(A, mc, sum, mx, arg);
   const int newp = (ctl.phase + 1) % 3;
-  double cl, cd;
-  clcd_block<R>(A, mc, newp, cl, cd);
-  __syncthreads();
+  // the control block is read here and written after the reduction's barrier
+  const int err = ctl.err, err_point = ctl.err_point;
+  const int row = ctl.hist_off + ctl.n_done % ctl.hist_cap;
+  const Moments v = mesh_moments<R>(A, mc, A.st[newp], 3);
+  const bool stopped = err != 0 || err_point != INT_MAX;
+  if (threadIdx.x == 32 && !stopped) {
+    const double cl = force_coefficient(mc, v, 0);
+    ctl.cl = cl;
+    A.h_cl[row] = cl;
+  }
+  if (threadIdx.x == 64 && !stopped) {
+    const double cd = force_coefficient(mc, v, 1);
+    ctl.cd = cd;
+    A.h_cd[row] = cd;
+  }
   if (threadIdx.x != 0) return;
   ctl.phase = newp;
   if (mc.iflow == 3) ctl.nphase = 1 - ctl.nphase;
-  if (ctl.err) {                            // roe_flux.f stop, inside residu
+  if (err) {                            // roe_flux.f stop, inside residu
     ctl.active = 0;
     return;
   }
-  if (ctl.err_point != INT_MAX) {          // check_positivity.f stop
+  if (err_point != INT_MAX) {          // check_positivity.f stop
     ctl.err = 3;
     ctl.active = 0;
     return;
   }
-  ctl.cl = cl;
-  ctl.cd = cd;
-  double fres = sqrt(sum / double(mc.nv));
-  ctl.fresi = mx;
-  ctl.iresi = (mx > 0.0) ? arg : 0;
+  double fres = residual_norm(mc, v);
+  ctl.fresi = v.m;
+  ctl.iresi = (v.m > 0.0) ? v.a : 0;
   if (ctl.iter == ctl.iterlast) {
     ctl.fres1 = fres;
     if (fres == 0.0) {
@@ -2023,16 +2067,11 @@ __global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A) 
       return;
     }
   }
-  fres = fres / ctl.fres1;
+  fres = div64(fres, ctl.fres1);
   ctl.fres = fres;
-  {
-    const int row = ctl.hist_off + ctl.n_done % ctl.hist_cap;
-    A.h_fres[row] = fres;
-    A.h_iresi[row] = ctl.iresi;
-    A.h_fresi[row] = ctl.fresi;
-    A.h_cl[row] = cl;
-    A.h_cd[row] = cd;
-  }
+  A.h_fres[row] = fres;
+  A.h_iresi[row] = ctl.iresi;
+  A.h_fresi[row] = v.m;
   ctl.iter += 1;
   ctl.n_done += 1;
   if (fres <= ctl.minres || ctl.n_done >= ctl.n_max) ctl.active = 0;
@@ -2148,18 +2187,16 @@ __global__ void __launch_bounds__(kBlockVerts) k_conres_part(ArenaPtrs<R> A) {
 
 // conres (first: set fres1) or clcd for one mesh, routine mode.
 template <typename R>
-__global__ void __launch_bounds__(256) k_routine_monitor(ArenaPtrs<R> A, int mesh, int what,
-                                                         int first) {
+__global__ void __launch_bounds__(kMonitorMaxThreads)
+    k_routine_monitor(ArenaPtrs<R> A, int mesh, int what, int first) {
   MeshCtl &ctl = A.ctl[mesh];
   const MeshConst &mc = A.mc[mesh];
+  const Moments v = mesh_moments<R>(A, mc, A.st[ctl.phase], what == 0 ? 1 : 2);
   if (what == 0) {
-    double sum, mx;
-    int arg;
-    conres_block<R>(A, mc, sum, mx, arg);
     if (threadIdx.x != 0) return;
-    double fres = sqrt(sum / double(mc.nv));
-    ctl.fresi = mx;
-    ctl.iresi = (mx > 0.0) ? arg : 0;
+    double fres = residual_norm(mc, v);
+    ctl.fresi = v.m;
+    ctl.iresi = (v.m > 0.0) ? v.a : 0;
     if (first) {
       ctl.fres1 = fres;
       if (fres == 0.0) {
@@ -2168,13 +2205,10 @@ __global__ void __launch_bounds__(256) k_routine_monitor(ArenaPtrs<R> A, int mes
         return;
       }
     }
-    ctl.fres = fres / ctl.fres1;
+    ctl.fres = div64(fres, ctl.fres1);
   } else {
-    double cl, cd;
-    clcd_block<R>(A, mc, ctl.phase, cl, cd);
-    if (threadIdx.x != 0) return;
-    ctl.cl = cl;
-    ctl.cd = cd;
+    if (threadIdx.x == 32) ctl.cl = force_coefficient(mc, v, 0);
+    if (threadIdx.x == 64) ctl.cd = force_coefficient(mc, v, 1);
   }
 }
 

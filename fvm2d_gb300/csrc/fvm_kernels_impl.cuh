@@ -209,7 +209,7 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_monitor(const ArenaPtrs<R> &A, const LaunchCfg &c) {                   \
     if (A.nslots <= 0) return cudaSuccess;                                                 \
-    k_monitor<KT<R>><<<A.nslots, monitor_threads<R>(), 0, c.stream>>>(kptrs(A));                      \
+    k_monitor<KT<R>><<<A.nslots, kMonitorMaxThreads, 0, c.stream>>>(kptrs(A));                      \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_update(const ArenaPtrs<R> &A, const LaunchCfg &c, int irk) {           \
@@ -226,11 +226,11 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_conres(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh, int first) {\
     k_conres_part<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                             \
-    k_routine_monitor<KT<R>><<<1, 256, 0, c.stream>>>(kptrs(A), mesh, 0, first);                       \
+    k_routine_monitor<KT<R>><<<1, kMonitorMaxThreads, 0, c.stream>>>(kptrs(A), mesh, 0, first);                       \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_clcd(const ArenaPtrs<R> &A, const LaunchCfg &c, int mesh) {             \
-    k_routine_monitor<KT<R>><<<1, 256, 0, c.stream>>>(kptrs(A), mesh, 1, 0);                           \
+    k_routine_monitor<KT<R>><<<1, kMonitorMaxThreads, 0, c.stream>>>(kptrs(A), mesh, 1, 0);                           \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_gradient_edge(const ArenaPtrs<R> &A, const LaunchCfg &c) {             \
