@@ -6,7 +6,8 @@
 // worth of vertices in sweep order form one half.  Splits alternate
 // direction by themselves, so the leaves (blocks of <= block_verts
 // vertices, consecutive in the new numbering) are compact patches and few
-// edges cross block boundaries.
+// edges cross block boundaries.  Inside a leaf the vertices follow the driver's
+// order.
 //
 // Block tables: the interior edges of iedge (residu.f:38-66) touching a
 // block, in iedge order; the solid then farfield edges of beindx
@@ -59,8 +60,12 @@ void sweep(const std::vector<int> &adj_ptr, const std::vector<int> &adj,
       if (B.seen[v] != s) visit_from(v);
 }
 
+// Leaves of at most bv vertices; inside a leaf, patches of at most pv vertices
+// (bv or a half or a quarter of it), each in ascending driver order: edges are
+// listed by driver vertex, so neighbouring lanes of an edge pass then touch
+// neighbouring vertices.
 void bisect(const std::vector<int> &adj_ptr, const std::vector<int> &adj, std::vector<int> verts,
-            int bv, Bfs &B, std::vector<int> &perm, std::vector<int> &block_start) {
+            int bv, int pv, Bfs &B, std::vector<int> &perm, std::vector<int> &block_start) {
   // explicit stack to bound recursion depth
   std::vector<std::vector<int>> stack;
   stack.push_back(std::move(verts));
@@ -73,13 +78,15 @@ void bisect(const std::vector<int> &adj_ptr, const std::vector<int> &adj, std::v
     sweep(adj_ptr, adj, part, part[part.size() / 2], part_stamp, B, order);
     const int root = order.back();
     sweep(adj_ptr, adj, part, root, part_stamp, B, order);
-    if ((int)part.size() <= bv) {
-      block_start.push_back((int)perm.size());
+    if ((int)part.size() <= pv) {
+      if (perm.size() % bv == 0) block_start.push_back((int)perm.size());
+      std::sort(order.begin(), order.end());
       perm.insert(perm.end(), order.begin(), order.end());
       continue;
     }
-    const int nblocks = ((int)part.size() + bv - 1) / bv;
-    const size_t nleft = size_t((nblocks + 1) / 2) * bv;
+    const int unit = (int)part.size() > bv ? bv : pv;
+    const int nunits = ((int)part.size() + unit - 1) / unit;
+    const size_t nleft = size_t((nunits + 1) / 2) * unit;
     std::vector<int> left(order.begin(), order.begin() + nleft);
     std::vector<int> right(order.begin() + nleft, order.end());
     // right is processed after left: push right first
@@ -91,7 +98,8 @@ void bisect(const std::vector<int> &adj_ptr, const std::vector<int> &adj, std::v
 }  // namespace
 
 void order_vertices(int np, const std::vector<int> &adj_ptr, const std::vector<int> &adj,
-                    int block_verts, std::vector<int> &perm, std::vector<int> &block_start) {
+                    int block_verts, int patch_verts, std::vector<int> &perm,
+                    std::vector<int> &block_start) {
   perm.clear();
   block_start.clear();
   if (np <= 0) return;
@@ -100,7 +108,7 @@ void order_vertices(int np, const std::vector<int> &adj_ptr, const std::vector<i
   B.inset.assign(np, 0);
   std::vector<int> all(np);
   for (int i = 0; i < np; i++) all[i] = i;
-  bisect(adj_ptr, adj, std::move(all), block_verts, B, perm, block_start);
+  bisect(adj_ptr, adj, std::move(all), block_verts, patch_verts, B, perm, block_start);
 }
 
 int32_t build_layout(const fvm_mesh &m, int bv, bool owned_first, MeshLayout &L) {
@@ -128,7 +136,11 @@ int32_t build_layout(const fvm_mesh &m, int bv, bool owned_first, MeshLayout &L)
     }
   }
   std::vector<int> block_start;
-  order_vertices(np, deg, adj, kBlockVerts, L.perm, block_start);
+  // FP64 (owned_first): compact patches of 64, the blocks a small mesh's leaves
+  // are split into; FP32: whole leaves in driver order (8 x 1024x384, chained
+  // iterations: breadth-first order 0.685 ms, patches of 64 0.673, leaves 0.664)
+  order_vertices(np, deg, adj, kBlockVerts, owned_first ? kBlockVerts / 4 : kBlockVerts, L.perm,
+                 block_start);
   // leaves split into blocks of bv consecutive vertices (the order, and so
   // every sum over vertices, is that of whole leaves)
   L.sub = kBlockVerts / bv;

@@ -57,8 +57,10 @@ int32_t build_layout(const fvm_mesh &m, int block_verts, bool owned_first, MeshL
 // every index inside its block's tiles); returns the number of violations.
 int64_t verify_layout(const MeshLayout &L);
 
-// Vertex order only (exposed for tests of the partitioner).
+// Vertex order only: leaves of block_verts vertices, made of patches of
+// patch_verts in ascending driver order.
 void order_vertices(int np, const std::vector<int> &adj_ptr, const std::vector<int> &adj,
-                    int block_verts, std::vector<int> &perm, std::vector<int> &block_start);
+                    int block_verts, int patch_verts, std::vector<int> &perm,
+                    std::vector<int> &block_start);
 
 }  // namespace fvm
