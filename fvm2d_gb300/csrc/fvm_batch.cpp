@@ -518,7 +518,6 @@ int32_t update_work(fvm_batch *b) {
   const bool use_fused = b->fused_wanted && b->fused_fits;
   changed |= use_fused != b->fused;
   b->fused = use_fused;
-  if (changed) drop_graphs(b);          // different kernels or tiles: re-capture
   const int n = (int)work.size();
   // the work list in kMaxChains parts at mesh boundaries: part k ends at
   // the boundary nearest (k+1)/chains of the list (the last parts are empty
@@ -537,6 +536,19 @@ int32_t update_work(fvm_batch *b) {
     head[k] = end;
     prev = end;
   }
+  // Chains side by side: a launch that fills the device makes the other
+  // chains' launches queue behind its persistent CTAs, so with four parts at
+  // work each takes half of the device and with seven or eight a third (the
+  // kernels then overlap from their start; grids of 912 / 456 / 304 CTAs, ms
+  // per iteration: 8 x 1024x384 in four chains 0.691 / 0.683 / 0.710, in eight
+  // 0.704 / 0.684 / 0.678; the 24-mesh mix in eight 0.796 / 0.750 / 0.722).
+  // Two or three parts measured best with whole waves.
+  int parts = 0;
+  for (int k = 1; k <= kMaxChains; k++) parts += head[k] > (k > 1 ? head[k - 1] : 0);
+  const int share = parts >= 7 ? 3 : parts >= 4 ? 2 : 1;
+  changed |= share != b->cfg.share;
+  b->cfg.share = share;
+  if (changed) drop_graphs(b);          // different kernels, tiles or grids: re-capture
   // the part (chain) of every resident mesh, for the per-chain monitors
   std::vector<int> part(b->slots.size(), 0);
   {
@@ -892,6 +904,7 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
     return fail(FVM_ERR_ARG);
   b->cfg.viscous = c.viscous != 0;
   b->cfg.std_const = false;   // set when meshes are admitted
+  b->cfg.share = 1;
   b->cfg.stream = b->stream;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);

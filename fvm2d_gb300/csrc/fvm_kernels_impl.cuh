@@ -42,7 +42,7 @@ inline int fit_grid(const LaunchCfg &c, K kern, size_t smem, int threads = kBloc
     (void)cudaGetLastError();
     occ = 1;
   }
-  const int g = (occ < 1 ? 1 : occ) * c.sms;
+  const int g = (occ < 1 ? 1 : occ) * c.sms / c.share;
   return g < c.grid ? g : c.grid;
 }
 

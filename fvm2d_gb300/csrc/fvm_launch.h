@@ -19,7 +19,8 @@ struct LaunchCfg {
   int max_tri2;      // max triangles of a block plus those of its halo
   int max_loc;       // max own + halo vertices of a block
   int sms;           // multiprocessors of the device
-  bool fit;          // grid = CTAs resident at once (occupancy x sms), capped by grid
+  bool fit;          // grid = CTAs resident at once (occupancy x sms) / share, capped by grid
+  int share;         // chains: the part of the device one launch takes (see update_work)
   int grad_mode;     // gradient pass: 1 loads per thread (k_grad), 2 per vertex
                      // (k_grad_v), 3 bulk copies to shared memory (k_grad_bulk, FP32)
   int max_halo;      // max halo vertices of a block (k_grad_bulk's halo ids)
