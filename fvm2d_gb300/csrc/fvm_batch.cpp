@@ -1522,6 +1522,35 @@ extern "C" int32_t fvm_batch_set_form(fvm_batch *b, int32_t form) {
   return apply_form(b, f);
 }
 
+// The best form's graphs so far, put aside while the tuner tries the others
+// and given back at its end: capturing and instantiating them again would fall
+// into the first step after it (10 iterations in eight chains: about 900
+// nodes, 15 ms).  What they hold (kernels, tiles, grids, parts) is the same when the
+// form is applied again, since no mesh comes or goes in between.
+struct KeptGraphs {
+  cudaGraphExec_t graph = nullptr, graph_multi = nullptr;
+  int kernels = 0, launches = 0;
+  void drop() {
+    if (graph) cudaGraphExecDestroy(graph);
+    if (graph_multi) cudaGraphExecDestroy(graph_multi);
+    graph = graph_multi = nullptr;
+  }
+  void take(fvm_batch *b) {   // after the form's timing: nothing of it is running
+    drop();
+    std::swap(graph, b->graph);
+    std::swap(graph_multi, b->graph_multi);
+    kernels = b->kernels_per_iter;
+    launches = b->launches_per_iter;
+  }
+  void give(fvm_batch *b) {
+    std::swap(graph, b->graph);
+    std::swap(graph_multi, b->graph_multi);
+    b->kernels_per_iter = kernels;
+    b->launches_per_iter = launches;
+  }
+  ~KeptGraphs() { drop(); }
+};
+
 extern "C" int32_t fvm_batch_tune(fvm_batch *b, int32_t iters, int32_t max, double *ms_per_iter,
                                   int32_t *choice) {
   if (b && b->pending) {   // deferred admissions first
@@ -1541,6 +1570,7 @@ extern "C" int32_t fvm_batch_tune(fvm_batch *b, int32_t iters, int32_t max, doub
   }
   int best = -1;
   double best_ms = 0.0;
+  KeptGraphs kept;
   int32_t st = FVM_OK;
   // every fourth call times every candidate; in between, a candidate more
   // than kTuneSkip times slower than the best of its last timing is not
@@ -1585,12 +1615,14 @@ extern "C" int32_t fvm_batch_tune(fvm_batch *b, int32_t iters, int32_t max, doub
     if (best < 0 || per < best_ms) {
       best = i;
       best_ms = per;
+      if (!b->timing) kept.take(b);   // (timed graphs carry events)
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (best < 0) best = form_fits(b, form_of(b, 0)) ? 0 : 1;
   const int32_t st2 = apply_form(b, form_of(b, best));
+  if (!st && !st2) kept.give(b);
   if (choice) *choice = best;
   return st ? st : st2;
 }
