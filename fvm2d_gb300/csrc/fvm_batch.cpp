@@ -546,6 +546,17 @@ int32_t update_work(fvm_batch *b) {
   int parts = 0;
   for (int k = 1; k <= kMaxChains; k++) parts += head[k] > (k > 1 ? head[k - 1] : 0);
   const int share = parts >= 7 ? 3 : parts >= 4 ? 2 : 1;
+  // FP64 edge pass: operations inlined while the edges fit one wave of its
+  // CTAs (4 x 128 per SM), where a warp's own latency counts; called above,
+  // where the warps wait for instructions.  us per iteration, inlined / called:
+  // 23k vertices (69k edges) Roe 219 / 254; 40k (119k edges) Roe 347 / 337, KFVS
+  // 404 / 387, HLLC 662 / 606; 98k laminar 901 / 871; 393k Roe 2417 / 2096.
+  int64_t edges = 0;
+  for (const Slot &s : b->slots)
+    if (s.used && !s.staged) edges += (int64_t)s.L.be_nodes.size();
+  const bool edge_calls = b->prec == FVM_PREC_FP64 && edges > (int64_t)b->cfg.sms * 4 * 128;
+  changed |= edge_calls != b->cfg.edge_calls;
+  b->cfg.edge_calls = edge_calls;
   changed |= share != b->cfg.share;
   b->cfg.share = share;
   if (changed) drop_graphs(b);          // different kernels, tiles or grids: re-capture
@@ -905,6 +916,7 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
   b->cfg.viscous = c.viscous != 0;
   b->cfg.std_const = false;   // set when meshes are admitted
   b->cfg.share = 1;
+  b->cfg.edge_calls = false;
   b->cfg.stream = b->stream;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);

@@ -21,12 +21,18 @@ namespace fvm {
 
 __device__ __forceinline__ float msqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double msqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ F64 msqrt(F64 x) { return F64(sqrt64(x.v)); }
-__device__ __forceinline__ F64 merf(F64 x) { return F64(erf(x.v)); }
-__device__ __forceinline__ F64 mexp(F64 x) { return F64(exp(x.v)); }
-__device__ __forceinline__ F64 mpow(F64 x, F64 y) { return F64(pow(x.v, y.v)); }
-__device__ __forceinline__ F64 mdiv(F64 a, F64 b) { return F64(div64(a.v, b.v)); }
-__device__ __forceinline__ F64 mfabs(F64 x) { return F64(fabs(x.v)); }
+template <int C>
+__device__ __forceinline__ F64T<C> msqrt(F64T<C> x) { return sqrt_as<C>(x.v); }
+template <int C>
+__device__ __forceinline__ F64T<C> merf(F64T<C> x) { return erf(x.v); }
+template <int C>
+__device__ __forceinline__ F64T<C> mexp(F64T<C> x) { return exp(x.v); }
+template <int C>
+__device__ __forceinline__ F64T<C> mpow(F64T<C> x, F64T<C> y) { return pow(x.v, y.v); }
+template <int C>
+__device__ __forceinline__ F64T<C> mdiv(F64T<C> a, F64T<C> b) { return div_as<C>(a.v, b.v); }
+template <int C>
+__device__ __forceinline__ F64T<C> mfabs(F64T<C> x) { return fabs(x.v); }
 __device__ __forceinline__ float merf(float x) { return erff(x); }
 __device__ __forceinline__ double merf(double x) { return erf(x); }
 // FP32: the fast hardware approximations (a few ulp), like the approximate
@@ -51,8 +57,8 @@ __device__ __forceinline__ R dmax1(R a, R b) { return b > a ? b : a; }
 // x > 0, dmin1(x, 0) (F64: from the bits)
 template <typename R>
 __device__ __forceinline__ bool positive(R x) { return x > R(0); }
-template <>
-__device__ __forceinline__ bool positive<F64>(F64 x) { return pos64(x.v); }
+template <int C>
+__device__ __forceinline__ bool positive(F64T<C> x) { return pos64(x.v); }
 template <typename R>
 __device__ __forceinline__ R min0(R x) { return positive(x) ? R(0) : x; }
 template <typename R>
@@ -61,16 +67,16 @@ __device__ __forceinline__ R sq(R x) { return x * x; }
 // rounds as the two would)
 template <typename R>
 __device__ __forceinline__ R half(R x) { return R(0.5) * x; }
-template <>
-__device__ __forceinline__ F64 half<F64>(F64 x) { return F64(half64(x.v)); }
+template <int C>
+__device__ __forceinline__ F64T<C> half(F64T<C> x) { return half64(x.v); }
 template <typename R>
 __device__ __forceinline__ R add_half(R p, R x) { return p + R(0.5) * x; }
-template <>
-__device__ __forceinline__ F64 add_half<F64>(F64 p, F64 x) { return F64(fma(0.5, x.v, p.v)); }
+template <int C>
+__device__ __forceinline__ F64T<C> add_half(F64T<C> p, F64T<C> x) { return fma(0.5, x.v, p.v); }
 template <typename R>
 __device__ __forceinline__ R sub_half(R p, R x) { return p - R(0.5) * x; }
-template <>
-__device__ __forceinline__ F64 sub_half<F64>(F64 p, F64 x) { return F64(fma(-0.5, x.v, p.v)); }
+template <int C>
+__device__ __forceinline__ F64T<C> sub_half(F64T<C> p, F64T<C> x) { return fma(-0.5, x.v, p.v); }
 template <typename R>
 __device__ __forceinline__ R cube(R x) { return (x * x) * x; }
 template <typename R>
@@ -130,6 +136,7 @@ __device__ __forceinline__ void recon1(R p1, R p2, R gx1, R gy1, R gx2, R gy2, R
 // F64: one side of the limited reconstruction, p + 0.5 s limit(ul, ur): ur2e =
 // ur^2 + eps.  The sign test of ul ur needs no product when both are inside
 // the window of exponents, where it cannot underflow.
+template <int C>
 __device__ __forceinline__ double limited_side(double p, double ul, double ur, double ur2,
                                                double ur2e, double eps, double s) {
   const uint32_t a = (uint32_t)__double2hiint(ul), b = (uint32_t)__double2hiint(ur);
@@ -138,15 +145,16 @@ __device__ __forceinline__ double limited_side(double p, double ul, double ur, d
   } else if ((int)(a ^ b) < 0) {
     return fma(s, 0.0, p);
   }
-  const double ul2 = mul64(ul, ul);
-  const double top = mul64(ul2 + eps, ur) + mul64(ur2e, ul);
+  const double ul2 = mul_as<C>(ul, ul);
+  const double top = mul_as<C>(ul2 + eps, ur) + mul_as<C>(ur2e, ul);
   const double bot = ul2 + ur2 + 2.0 * eps;
-  return fma(s, div64(top, bot), p);
+  return fma(s, div_as<C>(top, bot), p);
 }
 
 // recon.f:4-50 for one variable, FP64: recon1's operations, some products on
 // the FP64 pipe (which has room beside the sums), the others and the
 // quotients in integer arithmetic.
+template <int C>
 __device__ __forceinline__ void recon1_f64(double p1, double p2, double gx1, double gy1,
                                            double gx2, double gy2, double dx, double dy,
                                            int ilimit, double a11, double a12, double a21,
@@ -156,9 +164,9 @@ __device__ __forceinline__ void recon1_f64(double p1, double p2, double gx1, dou
     const double c = a22 * dqp;
     const double ul = a21 * (dx * gx1 + dy * gy1) + c;
     const double ur = a21 * (dx * gx2 + dy * gy2) + c;
-    const double q2 = mul64(dqp, dqp), q2e = q2 + eps;
-    pl = limited_side(p1, ul, dqp, q2, q2e, eps, 0.5);
-    pr = limited_side(p2, ur, dqp, q2, q2e, eps, -0.5);
+    const double q2 = mul_as<C>(dqp, dqp), q2e = q2 + eps;
+    pl = limited_side<C>(p1, ul, dqp, q2, q2e, eps, 0.5);
+    pr = limited_side<C>(p2, ur, dqp, q2, q2e, eps, -0.5);
   } else {
     const double c = a12 * dqp;
     pl = fma(0.5, a11 * (dx * gx1 + dy * gy1) + c, p1);
@@ -285,6 +293,79 @@ __device__ __forceinline__ bool roe_flux<float>(float ct, float st, float length
   flux[1] = (Fc1 + Fd1) * length;
   flux[2] = (Fc2 + Fd2) * length;
   flux[3] = (Fc3 + Fd3) * length;
+  return ok;
+}
+
+// FP64: roe_flux with its inputs in shared memory (face: rows of `stride`, left
+// rho, u, v, p, then right) and the central flux put back there (rows 8..11),
+// so that few values are live at a time: seven CTAs per SM fit
+// instead of four.
+template <int C>
+__device__ __forceinline__ bool roe_flux_f64(volatile double *face, int stride, F64T<C> ct,
+                                             F64T<C> st, F64T<C> length, F64T<C> GAMMA,
+                                             F64T<C> GAMMA1, F64T<C> flux[4]) {
+  using F64 = F64T<C>;
+  auto in = [&](int q) { return F64(face[q * stride]); };
+  auto put = [&](int q, F64 x) { face[q * stride] = x.v; };
+  F64 hl, hr, ql2, qr2;
+  {
+    const F64 rl = in(0), ul = in(1), vl = in(2), pl = in(3);
+    const F64 al2 = mdiv(GAMMA * pl, rl);
+    ql2 = sq(ul) + sq(vl);
+    hl = add_half(mdiv(al2, GAMMA1), ql2);
+    const F64 unl = ul * ct + vl * st;
+    put(8, rl * unl);
+    put(9, pl * ct + rl * ul * unl);
+    put(10, pl * st + rl * vl * unl);
+    put(11, rl * hl * unl);
+  }
+  {
+    const F64 rr = in(4), ur = in(5), vr = in(6), pr = in(7);
+    const F64 ar2 = mdiv(GAMMA * pr, rr);
+    qr2 = sq(ur) + sq(vr);
+    hr = add_half(mdiv(ar2, GAMMA1), qr2);
+  }
+  F64 ua, va, ha;
+  {
+    const F64 rl12 = msqrt(in(0)), rr12 = msqrt(in(4));
+    const F64 rd = mdiv(F64(1.0), rl12 + rr12);
+    ua = (in(1) * rl12 + in(5) * rr12) * rd;
+    va = (in(2) * rl12 + in(6) * rr12) * rd;
+    ha = (hl * rl12 + hr * rr12) * rd;
+  }
+  const F64 qa2 = sq(ua) + sq(va);
+  const F64 aa2 = GAMMA1 * sub_half(ha, qa2);
+  const bool ok = positive(aa2);
+  const F64 aa = msqrt(aa2);
+  const F64 una = ua * ct + va * st;
+  const F64 vna = -ua * st + va * ct;
+  F64 a1l1, a2l2, a3l3, a4l4;
+  {
+    const F64 rl = in(0), rr = in(4);
+    const F64 du1 = rr - rl;
+    const F64 du2 = rr * in(5) - rl * in(1);
+    const F64 du3 = rr * in(6) - rl * in(2);
+    const F64 du4 = add_half(mdiv(in(7) - in(3), GAMMA1), rr * qr2 - rl * ql2);
+    const F64 m1 = mdiv(ct * du2 + st * du3 - una * du1, aa);
+    const F64 m2 = mdiv(GAMMA1 * (du4 - ua * du2 - va * du3 + qa2 * du1), sq(aa));
+    const F64 a4 = half(m1 + m2);
+    const F64 a1 = half(m2 - m1);
+    const F64 a3 = du1 - a1 - a4;
+    const F64 a2 = mdiv(st * du2 - ct * du3 + vna * du1, aa);
+    const F64 l2 = min0(una);
+    a1l1 = a1 * min0(una - aa);
+    a2l2 = a2 * l2;
+    a3l3 = a3 * l2;
+    a4l4 = a4 * min0(una + aa);
+  }
+  const F64 aact = aa * ct, aast = aa * st;
+  const F64 a2a = a2l2 * aa;
+  flux[0] = (in(8) + (a1l1 + a3l3 + a4l4)) * length;
+  flux[1] = (in(9) + (a1l1 * (ua - aact) + a2a * st + a3l3 * ua + a4l4 * (ua + aact))) * length;
+  flux[2] = (in(10) + (a1l1 * (va - aast) - a2a * ct + a3l3 * va + a4l4 * (va + aast))) * length;
+  const F64 unaa = una * aa;
+  flux[3] = (in(11) + (a1l1 * (ha - unaa) + a2a * vna + half(a3l3) * qa2 + a4l4 * (ha + unaa))) *
+            length;
   return ok;
 }
 

@@ -234,27 +234,41 @@ FVM_I64 bool pos64(double a) {
   return u - 1u < 0x7ff0000000000000ull;
 }
 
+// The operations inlined (C = 0) or as functions (C = 1).  Inlined they are the
+// quicker way for a warp alone; but long kernels of them wait for their own
+// instructions once many warps stream through the code (16 bytes per
+// instruction), and functions stay in the nearest instruction cache.
+FVM_I64_CALL double i64_mul_call(double a, double b) { return mul64(a, b); }
+FVM_I64_CALL double i64_div_call(double a, double b) { return div64(a, b); }
+FVM_I64_CALL double i64_sqrt_call(double a) { return sqrt64(a); }
+template <int C>
+FVM_I64 double mul_as(double a, double b) { return C ? i64_mul_call(a, b) : mul64(a, b); }
+template <int C>
+FVM_I64 double div_as(double a, double b) { return C ? i64_div_call(a, b) : div64(a, b); }
+template <int C>
+FVM_I64 double sqrt_as(double a) { return C ? i64_sqrt_call(a) : sqrt64(a); }
+
 // A double whose products, quotients and square roots are the ones above and
 // whose sums are the FP64 pipe's; the arithmetic of fvm_device.cuh compiles
-// for it as for double.  The / operator calls a function (shorter code: the
-// HLLC flux, which divides 25 times, 639 -> 597 us on 768 x 256), mdiv is
-// inlined.
-struct F64 {
+// for it as for double.  The / operator always calls (the HLLC flux, which
+// divides 25 times, 639 -> 597 us on 768 x 256), mdiv follows C.
+template <int C>
+struct F64T {
   double v;
-  F64() = default;
-  FVM_I64 F64(double x) : v(x) {}
+  F64T() = default;
+  FVM_I64 F64T(double x) : v(x) {}
   FVM_I64 explicit operator double() const { return v; }
+  FVM_I64 friend F64T operator+(F64T a, F64T b) { return F64T(a.v + b.v); }
+  FVM_I64 friend F64T operator-(F64T a, F64T b) { return F64T(a.v - b.v); }
+  FVM_I64 friend F64T operator-(F64T a) { return F64T(-a.v); }
+  FVM_I64 friend F64T operator*(F64T a, F64T b) { return F64T(mul_as<C>(a.v, b.v)); }
+  FVM_I64 friend F64T operator/(F64T a, F64T b) { return F64T(i64_div_call(a.v, b.v)); }
+  FVM_I64 friend bool operator<(F64T a, F64T b) { return a.v < b.v; }
+  FVM_I64 friend bool operator>(F64T a, F64T b) { return a.v > b.v; }
+  FVM_I64 friend bool operator<=(F64T a, F64T b) { return a.v <= b.v; }
+  FVM_I64 friend bool operator>=(F64T a, F64T b) { return a.v >= b.v; }
+  FVM_I64 friend bool operator!=(F64T a, F64T b) { return a.v != b.v; }
 };
-FVM_I64 F64 operator+(F64 a, F64 b) { return F64(a.v + b.v); }
-FVM_I64 F64 operator-(F64 a, F64 b) { return F64(a.v - b.v); }
-FVM_I64 F64 operator-(F64 a) { return F64(-a.v); }
-FVM_I64 F64 operator*(F64 a, F64 b) { return F64(mul64(a.v, b.v)); }
-FVM_I64_CALL double i64_div_call(double a, double b) { return div64(a, b); }
-FVM_I64 F64 operator/(F64 a, F64 b) { return F64(i64_div_call(a.v, b.v)); }
-FVM_I64 bool operator<(F64 a, F64 b) { return a.v < b.v; }
-FVM_I64 bool operator>(F64 a, F64 b) { return a.v > b.v; }
-FVM_I64 bool operator<=(F64 a, F64 b) { return a.v <= b.v; }
-FVM_I64 bool operator>=(F64 a, F64 b) { return a.v >= b.v; }
-FVM_I64 bool operator!=(F64 a, F64 b) { return a.v != b.v; }
+using F64 = F64T<0>;
 
 }  // namespace fvm

@@ -32,6 +32,9 @@
 #ifndef FVM_EFLUX_MINB
 #define FVM_EFLUX_MINB 4    // resident CTAs per SM asked of the FP64 edge kernel (5-8: 3-8% slower)
 #endif
+#ifndef FVM_EFLUX_CALLB
+#define FVM_EFLUX_CALLB 7   // the same with called operations (5, 6: 2-12% slower, 8: the same)
+#endif
 #ifndef FVM_GATHER_BATCH
 #define FVM_GATHER_BATCH 1  // FP32 flux pass: incidences loaded together in the per-vertex gather
 #endif
@@ -1075,10 +1078,11 @@ __device__ __forceinline__ void edge_flux_f32(const ArenaPtrs<float> &A, const F
 // thread's column): integer arithmetic makes long code, and unrolled the pass
 // waited for instructions a quarter of the time.
 constexpr int kEdgeThreads = 128;
-template <int FLUX>
-__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<F64> &A, const FluxConst<F64> &fc,
-                                              const R4<F64> *P, int e, double *face, F64 f[4],
+template <int FLUX, int C>
+__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<F64> &A, const MeshConst &mc,
+                                              const R4<F64> *P, int e, double *face, F64T<C> f[4],
                                               int &err) {
+  using T = F64T<C>;
   const int2 nn = A.be_nodes[e];
   const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
   const double dx = c2.x - c1.x, dy = c2.y - c1.y;
@@ -1089,19 +1093,24 @@ __device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<F64> &A, const Flu
 #pragma unroll 1
   for (int q = 0; q < 4; q++) {
     double pl, pr;
-    recon1_f64(s1[q], s2[q], g1[q], g1[4 + q], g2[q], g2[4 + q], dx, dy, fc.ilimit, fc.a11.v,
-               fc.a12.v, fc.a21.v, fc.a22.v, fc.eps.v, pl, pr);
+    recon1_f64<C>(s1[q], s2[q], g1[q], g1[4 + q], g2[q], g2[4 + q], dx, dy, mc.ilimit,
+                  mc.albada11, mc.albada12, mc.albada21, mc.albada22, mc.epsilon, pl, pr);
     face[q * kEdgeThreads] = pl;
     face[(4 + q) * kEdgeThreads] = pr;
   }
   const D4 csl = A.be_csl[e];
-  F64 pl[4], pr[4];
+  const FluxConst<T> fc = flux_const<T>(mc);
+  if constexpr (FLUX == 1) {
+    if (!roe_flux_f64<C>(face, kEdgeThreads, csl.x, csl.y, csl.z, fc.gamma, fc.gamma1, f)) err = 1;
+    return;
+  }
+  T pl[4], pr[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     pl[q] = face[q * kEdgeThreads];
     pr[q] = face[(4 + q) * kEdgeThreads];
   }
-  if (!riemann<F64, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f)) err = 1;
+  if (!riemann<T, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f)) err = 1;
 }
 
 // One boundary edge: its contributions to n1 and n2.
@@ -1285,15 +1294,18 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // cut edges in both blocks (+10%) and left most SMs idle in its last wave:
 // 1365 us for 1024 x 384, Roe; 1000 us here on the FP64 pipe alone (446
 // operations per edge at 526 Gop/s) and 149 us in the gather; 560 and 103 us
-// with the products, quotients and roots on the integer pipes (F64).  Now
-// neither pipe is full (FP64 57%, ALU 30%, issue 30%): 15 warps per SM wait
-// for each other's results and for instructions.  HLLC on 768 x 256: 1064 ->
-// 597 us, its pow still on the FP64 pipe.
-template <typename R, int FLUX>
-__global__ void __launch_bounds__(kEdgeThreads, FVM_EFLUX_MINB)
+// with the products, quotients and roots on the integer pipes (F64).  Neither
+// pipe was full then (FP64 57%, ALU 30%, issue 30%): the warps waited for
+// instructions, of which one edge takes 5800 (93 KB).  C = 1 calls the
+// operations instead of inlining them, and few live values (the reconstructed
+// states and the central flux wait in shared memory) let seven CTAs share an
+// SM: 442 us; the rule is in update_work.  HLLC on 768 x 256: 1064 -> 560 us,
+// its pow still on the FP64 pipe.
+template <typename R, int FLUX, int C>
+__global__ void __launch_bounds__(kEdgeThreads, C ? FVM_EFLUX_CALLB : FVM_EFLUX_MINB)
     k_eflux(ArenaPtrs<R> A, int stage, int routine, int items) {
   static_assert(sizeof(R) == 8, "the FP64 pass");
-  __shared__ double s_face[8 * kEdgeThreads];
+  __shared__ double s_face[(FLUX == 1 ? 12 : 8) * kEdgeThreads];
   int w0, nwork;
   work_range(A, w0, nwork);
   for (int i = w0 * items + blockIdx.x; i < nwork * items; i += gridDim.x) {
@@ -1311,13 +1323,13 @@ __global__ void __launch_bounds__(kEdgeThreads, FVM_EFLUX_MINB)
     const int k = c * kEdgeThreads + threadIdx.x;
     if (k >= A.blk_neo[bi.part]) continue;
     int err = 0;
-    R f[4];
-    edge_flux_f64<FLUX>(A, flux_const<R>(mc), P, bi.e0 + k, s_face + threadIdx.x, f, err);
+    F64T<C> f[4];
+    edge_flux_f64<FLUX, C>(A, mc, P, bi.e0 + k, s_face + threadIdx.x, f, err);
     R4<R> o;
-    o.x = f[0];
-    o.y = f[1];
-    o.z = f[2];
-    o.w = f[3];
+    o.x = f[0].v;
+    o.y = f[1].v;
+    o.z = f[2].v;
+    o.w = f[3].v;
     A.eflux[bi.e0 + k] = o;
     if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
   }

@@ -60,8 +60,12 @@ inline void launch_flux_code(const ArenaPtrs<R> &A, const LaunchCfg &c, int stag
     const int items = (c.max_slots + kEdgeThreads - 1) / kEdgeThreads + 1;
     LaunchCfg ce = c;
     ce.grid = c.grid > INT_MAX / items ? INT_MAX : c.grid * items;
-    k_eflux<KT<R>, F><<<fit_grid(ce, k_eflux<KT<R>, F>, 0, kEdgeThreads), kEdgeThreads, 0, c.stream>>>(
-        kptrs(A), stage, routine, items);
+    if (c.edge_calls)
+      k_eflux<KT<R>, F, 1><<<fit_grid(ce, k_eflux<KT<R>, F, 1>, 0, kEdgeThreads), kEdgeThreads, 0,
+                             c.stream>>>(kptrs(A), stage, routine, items);
+    else
+      k_eflux<KT<R>, F, 0><<<fit_grid(ce, k_eflux<KT<R>, F, 0>, 0, kEdgeThreads), kEdgeThreads, 0,
+                             c.stream>>>(kptrs(A), stage, routine, items);
     k_egather<KT<R>><<<fit_grid(c, k_egather<KT<R>>, 0), kBlockVerts, 0, c.stream>>>(kptrs(A), stage, mode, irk,
                                                                              routine);
   }
