@@ -23,6 +23,15 @@
 #ifndef FVM_GRAD_MINB32
 #define FVM_GRAD_MINB32 5   // resident CTAs per SM asked of the FP32 gradient kernel
 #endif
+#ifndef FVM_EGATHER_MINB
+#define FVM_EGATHER_MINB 4   // resident CTAs per SM asked of the FP64 gather kernel (2, 3: 10-30% slower)
+#endif
+#ifndef FVM_EGATHER_BATCH
+#define FVM_EGATHER_BATCH 2  // its incidences loaded together (4, 8 at fewer CTAs: 10-40% slower)
+#endif
+#ifndef FVM_GRAD_MINB64
+#define FVM_GRAD_MINB64 4   // the same of the FP64 one for inviscid meshes (3, 5: the same)
+#endif
 #ifndef FVM_GRADV_MINB32
 #define FVM_GRADV_MINB32 4  // the same for its per-vertex form
 #endif
@@ -379,8 +388,32 @@ __device__ __forceinline__ void grad_vertex_sums(const uint16_t *vtl, int j0, in
   }
 }
 
+// FP64, inviscid meshes: the sums of the four variables one after another (the
+// integer products make long code), the triangle sums as rows of max_tri in
+// shared memory, s[2 q] and s[2 q + 1] of variable q (random 64-byte records
+// conflict in the banks).  Few live values: four CTAs share an SM instead of
+// two; 136 -> 107 us on 1024 x 384.
 template <typename R>
-__global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 : 2)
+__device__ __forceinline__ void tri_sums_rows(const ArenaPtrs<R> &A, const R4<R> *P, int entry,
+                                              int k, R *s, int max_tri) {
+  const int4 t = A.bt_nodes[entry];
+  const R *s1 = reinterpret_cast<const R *>(P + t.x), *s2 = reinterpret_cast<const R *>(P + t.y),
+          *s3 = reinterpret_cast<const R *>(P + t.z);
+  R dbxx[3], dbyy[3];
+  tri_geom<R>(A, t, entry, dbxx, dbyy);
+#pragma unroll 1
+  for (int q = 0; q < 4; q++) {
+    const R a1 = s1[q], a2 = s2[q], a3 = s3[q];
+    s[2 * q * max_tri + k] = a1 * dbxx[0] + a2 * dbxx[1] + a3 * dbxx[2];
+    s[(2 * q + 1) * max_tri + k] = a1 * dbyy[0] + a2 * dbyy[1] + a3 * dbyy[2];
+  }
+}
+
+// VISC: viscous meshes may be among the blocks
+template <typename R, bool VISC>
+__global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32
+                                               : VISC         ? 2
+                                                              : FVM_GRAD_MINB64)
     k_grad(ArenaPtrs<R> A, int stage, int do_dt,
                                                       int routine, int max_tri, int skip_inviscid) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -394,7 +427,8 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 
     if (!routine && !ctl.active) continue;
     const MeshConst &mc = A.mc[bi.mesh];
     if (skip_inviscid && mc.iflow == 1) continue;   // the stencil pass's meshes
-    const bool visc = mc.iflow != 1;
+    const bool visc = VISC && mc.iflow != 1;
+    constexpr bool rows = sizeof(R) == 8 && !VISC;
     const R4<R> *P = A.st[cur_buf(ctl.phase, stage)];
     if (threadIdx.x == 0) {
       const BlockInfo *nb = next_block(A, w, nwork);
@@ -410,6 +444,10 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 
     }
     // phase 1: one thread per triangle touching the block
     for (int k = threadIdx.x; k < bi.nt; k += blockDim.x) {
+      if constexpr (rows) {
+        tri_sums_rows<R>(A, P, bi.t0 + k, k, reinterpret_cast<R *>(smem_raw), max_tri);
+        continue;
+      }
       const int4 t = A.bt_nodes[bi.t0 + k];
       const R4<R> p1 = P[t.x], p2 = P[t.y], p3 = P[t.z];
       R dbxx[3], dbyy[3];
@@ -430,9 +468,23 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 
       const int v = bi.v0 + threadIdx.x;
       R qx[4], qy[4], rv[3];
       const int2 jr = A.vt_rng[v];
-      // (FP32: one triangle at a time, the 48 registers of five CTAs per SM)
-      grad_vertex_sums<R, sizeof(R) == 8 ? 2 : 1>(A.vt_list, jr.x, jr.y, s_tri,
-                                                  visc ? s_vis : nullptr, qx, qy, rv);
+      if constexpr (rows) {
+        const R *s = reinterpret_cast<const R *>(smem_raw);
+#pragma unroll
+        for (int q = 0; q < 4; q++) qx[q] = qy[q] = R(0);
+        for (int j = jr.x; j < jr.y; j++) {
+          const R *e = s + (A.vt_list[j] & 0x3fff);
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            qx[q] = qx[q] + e[2 * q * max_tri];
+            qy[q] = qy[q] + e[(2 * q + 1) * max_tri];
+          }
+        }
+      } else {
+        // (FP32: one triangle at a time, the 48 registers of five CTAs per SM)
+        grad_vertex_sums<R, sizeof(R) == 8 ? 2 : 1>(A.vt_list, jr.x, jr.y, s_tri,
+                                                    visc ? s_vis : nullptr, qx, qy, rv);
+      }
       const R ais = v_ais(A, v);
       Grad<R> g;
 #pragma unroll
@@ -1185,8 +1237,7 @@ __device__ __forceinline__ void flux_boundary(const ArenaPtrs<R> &A, const MeshC
 }
 
 // Adds one incidence's flux to a vertex's residual.
-template <typename R>
-__device__ __forceinline__ void add_flux(R acc[4], uint16_t e, const R4<R> &f) {
+__device__ __forceinline__ void add_flux(float acc[4], uint16_t e, const R4<float> &f) {
   if (e & kSolidBit) {
     acc[1] = acc[1] + f.y;
     acc[2] = acc[2] + f.z;
@@ -1201,6 +1252,20 @@ __device__ __forceinline__ void add_flux(R acc[4], uint16_t e, const R4<R> &f) {
     acc[2] = acc[2] + f.z;
     acc[3] = acc[3] + f.w;
   }
+}
+// FP64: one addition per component whatever the sign (a warp whose lanes
+// differ would pass the FP64 pipe once for each; gather of 1024 x 384: 103 ->
+// 62 us together with the loads' batches): the sign bit is flipped first.  A solid edge's first and last component are +0, which changes no sum
+// (sums start at +0 and so are never -0).
+__device__ __forceinline__ F64 signed_by(F64 x, uint32_t sign) {
+  return F64(__hiloint2double((int)((uint32_t)__double2hiint(x.v) ^ sign), __double2loint(x.v)));
+}
+__device__ __forceinline__ void add_flux(F64 acc[4], uint16_t e, const R4<F64> &f) {
+  const uint32_t sign = (uint32_t)(e & kNegBit) << 16;
+  acc[0] = acc[0] + signed_by(f.x, sign);
+  acc[1] = acc[1] + signed_by(f.y, sign);
+  acc[2] = acc[2] + signed_by(f.z, sign);
+  acc[3] = acc[3] + signed_by(f.w, sign);
 }
 
 // Phase 2 of the flux pass: one thread per vertex sums its edge fluxes in
@@ -1231,8 +1296,9 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
     }
     const int2 jr = A.ve_rng[v];
     // GB incidences' slots and fluxes loaded together, then added in list
-    // order (FP64: the loads reach L2, four hide their latency)
-    constexpr int GB = sizeof(R) == 4 ? FVM_GATHER_BATCH : 4;
+    // order (FP64: the loads reach L2; two at four CTAs per SM hide their latency
+    // best)
+    constexpr int GB = sizeof(R) == 4 ? FVM_GATHER_BATCH : FVM_EGATHER_BATCH;
     for (int j = jr.x; j < jr.y; j += GB) {
       uint16_t es[GB];
       R4<R> fs[GB];
@@ -1253,7 +1319,7 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 #pragma unroll
       for (int u = 0; u < GB; u++) {
         if (j + u >= jr.y) break;
-        add_flux<R>(acc, es[u], fs[u]);
+        add_flux(acc, es[u], fs[u]);
       }
     }
     if (mode == MODE_RESIDUAL) {
@@ -1337,7 +1403,7 @@ __global__ void __launch_bounds__(kEdgeThreads, C ? FVM_EFLUX_CALLB : FVM_EFLUX_
 
 // FP64 flux pass, second kernel: gather per vertex and RK stage.
 template <typename R>
-__global__ void __launch_bounds__(kBlockVerts, 2)
+__global__ void __launch_bounds__(kBlockVerts, FVM_EGATHER_MINB)
     k_egather(ArenaPtrs<R> A, int stage, int mode, int irk, int routine) {
   __shared__ double s_red[kBlockVerts / 32], s_max[kBlockVerts / 32];
   __shared__ int s_arg[kBlockVerts / 32];

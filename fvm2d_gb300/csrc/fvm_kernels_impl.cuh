@@ -177,7 +177,13 @@ inline cudaError_t flux_attributes(size_t f) {
           kptrs(A), stage, do_dt, routine, c.max_tri, c.max_halo, c.viscous ? 1 : 0, skip);       \
       return cudaGetLastError();                                                           \
     }                                                                                      \
-    k_grad<KT<R>><<<fit_grid(c, k_grad<KT<R>>, sm), kBlockVerts, sm, c.stream>>>(kptrs(A), stage, do_dt, routine, c.max_tri, skip);  \
+    /* FP32: viscous meshes alone reach this form */                                       \
+    if (sizeof(R) == 4 || c.viscous)                                                       \
+      k_grad<KT<R>, true><<<fit_grid(c, k_grad<KT<R>, true>, sm), kBlockVerts, sm, c.stream>>>( \
+          kptrs(A), stage, do_dt, routine, c.max_tri, skip);                               \
+    else                                                                                   \
+      k_grad<KT<R>, (sizeof(R) == 4)><<<fit_grid(c, k_grad<KT<R>, (sizeof(R) == 4)>, sm), kBlockVerts, sm, c.stream>>>( \
+          kptrs(A), stage, do_dt, routine, c.max_tri, skip);                               \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_flux(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,   \
@@ -265,8 +271,11 @@ inline cudaError_t flux_attributes(size_t f) {
       if (k == 3) e2 = cudaFuncSetAttribute(k_step<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
       if (e2 != cudaSuccess) return e2;                                                    \
     }                                                                                      \
-    cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>>,                                        \
+    cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>, true>,                              \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g); \
+    if (e == cudaSuccess)                                                                  \
+      e = cudaFuncSetAttribute(k_grad<KT<R>, (sizeof(R) == 4)>,                      \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g);       \
     if (e == cudaSuccess) e = flux_attributes<R>(f);                                       \
     if (e == cudaSuccess)                                                                  \
       e = cudaFuncSetAttribute(k_sa<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s); \
