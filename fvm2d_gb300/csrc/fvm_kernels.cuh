@@ -1109,9 +1109,16 @@ __device__ __forceinline__ bool riemann(const FluxConst<T> &fc, T ct, T st, T le
 // FP32: the flux of edge entry e with ends nn (24 bytes per entry: the ends,
 // edge vector and ds; ds/|ds| and |ds| are formed after the reconstruction).
 // The records are read once a pass, by streaming loads that leave the caches to
-// the states and gradients (5 x 394x151 HLLC in eight chains 0.0938 -> 0.0901
-// ms per iteration, 8 x 1024x384 0.650 -> 0.646; the stencil's lists, whose
-// lines neighbouring trips share, get slower with them: 0.080 -> 0.115).
+// the states and gradients (5 x 394x151 HLLC in eight chains 0.0941 -> 0.0917
+// ms per iteration, 8 x 1024x384 0.656 -> 0.645; the stencil's lists, whose
+// lines neighbouring trips share, get slower with them: 0.080 -> 0.115).  The
+// ends' load is not volatile: ordered against the others it changed which of
+// the HLLC flux's products are contracted, and so its last bits.
+__device__ __forceinline__ int2 load_ends(const int2 *p) {
+  int2 r;
+  asm("ld.global.cs.v2.s32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  return r;
+}
 template <int FLUX>
 __device__ __forceinline__ void edge_flux_f32(const ArenaPtrs<float> &A, const FluxConst<float> &fc,
                                               const R4<float> *P, int e, int2 nn, float f[4],
@@ -1449,13 +1456,13 @@ __global__ void __launch_bounds__(kFluxThreads, FVM_FLUX_MINB32)
     // entry's states and gradients are in flight
 #if FVM_FLUX_PIPE
     int2 nn_next = make_int2(0, 0);
-    if (threadIdx.x < bi.ne) nn_next = __ldcs(A.be_nodes + bi.e0 + threadIdx.x);
+    if (threadIdx.x < bi.ne) nn_next = load_ends(A.be_nodes + bi.e0 + threadIdx.x);
 #endif
     for (int k = threadIdx.x; k < bi.ne; k += blockDim.x) {
       R f[4];
 #if FVM_FLUX_PIPE
       const int2 nn = nn_next;
-      if (k + (int)blockDim.x < bi.ne) nn_next = __ldcs(A.be_nodes + bi.e0 + k + blockDim.x);
+      if (k + (int)blockDim.x < bi.ne) nn_next = load_ends(A.be_nodes + bi.e0 + k + blockDim.x);
 #else
       const int2 nn = A.be_nodes[bi.e0 + k];
 #endif
