@@ -551,12 +551,22 @@ int32_t update_work(fvm_batch *b) {
   // where the warps wait for instructions.  us per iteration, inlined / called:
   // 23k vertices (69k edges) Roe 219 / 254; 40k (119k edges) Roe 347 / 337, KFVS
   // 404 / 387, HLLC 662 / 606; 98k laminar 901 / 871; 393k Roe 2417 / 2096.
-  int64_t edges = 0;
-  for (const Slot &s : b->slots)
-    if (s.used && !s.staged) edges += (int64_t)s.L.be_nodes.size();
-  const bool edge_calls = b->prec == FVM_PREC_FP64 && edges > (int64_t)b->cfg.sms * 4 * 128;
-  changed |= edge_calls != b->cfg.edge_calls;
-  b->cfg.edge_calls = edge_calls;
+  // Few edges, the items of four warps to 32 edges in one wave (6 CTAs per SM):
+  // a variable to a warp and products on the FP64 pipe.  us per iteration, thread
+  // per edge / four warps: 1.5k vertices Roe 136 / 105, KFVS 137 / 109; 7.7k Roe
+  // 173 / 135; 8k laminar 220 / 202; with two waves 12k Roe 166 / 180, HLLC 287 /
+  // 312.
+  int64_t edges = 0, few_items = 0;
+  for (const Slot &s : b->slots) {
+    if (!s.used || s.staged) continue;
+    edges += (int64_t)s.L.be_nodes.size();
+    for (int neo : s.L.neo) few_items += (neo + 31) / 32 + 1;
+  }
+  int edge_form = edges > (int64_t)b->cfg.sms * 4 * 128 ? 1 : 0;
+  if (few_items <= (int64_t)b->cfg.sms * 6) edge_form = 2;
+  if (b->prec != FVM_PREC_FP64) edge_form = 0;
+  changed |= edge_form != b->cfg.edge_form;
+  b->cfg.edge_form = edge_form;
   changed |= share != b->cfg.share;
   b->cfg.share = share;
   if (changed) drop_graphs(b);          // different kernels, tiles or grids: re-capture
@@ -916,7 +926,7 @@ extern "C" int32_t fvm_batch_create(int32_t precision, const fvm_batch_caps *cap
   b->cfg.viscous = c.viscous != 0;
   b->cfg.std_const = false;   // set when meshes are admitted
   b->cfg.share = 1;
-  b->cfg.edge_calls = false;
+  b->cfg.edge_form = 0;
   b->cfg.stream = b->stream;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);

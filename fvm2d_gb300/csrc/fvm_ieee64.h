@@ -237,12 +237,15 @@ FVM_I64 bool pos64(double a) {
 // The operations inlined (C = 0) or as functions (C = 1).  Inlined they are the
 // quicker way for a warp alone; but long kernels of them wait for their own
 // instructions once many warps stream through the code (16 bytes per
-// instruction), and functions stay in the nearest instruction cache.
+// instruction), and functions stay in the nearest instruction cache.  C = 2:
+// products on the FP64 pipe, for work so little that the pipe is never full.
 FVM_I64_CALL double i64_mul_call(double a, double b) { return mul64(a, b); }
 FVM_I64_CALL double i64_div_call(double a, double b) { return div64(a, b); }
 FVM_I64_CALL double i64_sqrt_call(double a) { return sqrt64(a); }
 template <int C>
-FVM_I64 double mul_as(double a, double b) { return C ? i64_mul_call(a, b) : mul64(a, b); }
+FVM_I64 double mul_as(double a, double b) {
+  return C == 2 ? a * b : C ? i64_mul_call(a, b) : mul64(a, b);
+}
 template <int C>
 FVM_I64 double div_as(double a, double b) { return C ? i64_div_call(a, b) : div64(a, b); }
 template <int C>

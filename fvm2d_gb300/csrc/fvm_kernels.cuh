@@ -41,6 +41,9 @@
 #ifndef FVM_EFLUX_MINB
 #define FVM_EFLUX_MINB 4    // resident CTAs per SM asked of the FP64 edge kernel (5-8: 3-8% slower)
 #endif
+#ifndef FVM_EFLUX_FEWB
+#define FVM_EFLUX_FEWB 6    // the same with four warps to 32 edges (4: 20%, 7: 9% slower at 160 x 48)
+#endif
 #ifndef FVM_EFLUX_CALLB
 #define FVM_EFLUX_CALLB 7   // the same with called operations (5, 6: 2-12% slower, 8: the same)
 #endif
@@ -1132,44 +1135,64 @@ __device__ __forceinline__ void edge_flux_f32(const ArenaPtrs<float> &A, const F
   if (!riemann<float, FLUX>(fc, ct, st, len, pl, pr, f)) err = 1;
 }
 
-// FP64: the flux of edge entry e.  The four variables' reconstructions are one
-// loop, its results in shared memory (`face`: 8 rows of kEdgeThreads, this
-// thread's column): integer arithmetic makes long code, and unrolled the pass
-// waited for instructions a quarter of the time.
+// FP64: the flux of edge entries.  The reconstructed states go through shared
+// memory (`face`: left rho, u, v, p, then right, then room for the Riemann
+// solver's central flux, each a row of `stride`).
+//
+// A thread per edge (C = 0, 1), the four variables one after another (unrolled,
+// the integer arithmetic made the pass wait for instructions a quarter of the
+// time), or, for few edges (C = 2), four warps to 32 edges, each warp
+// reconstructing one variable and the first solving the Riemann problems: a
+// launch then lasts as long as one edge's chain of operations, which is a
+// variable's and the solver's, and its code, with products on the FP64 pipe,
+// a fifth as long.  160 x 48, Roe: 33 us a thread per edge, 34 us four warps with
+// integer products (both fetch 93 KB of code), 21.5 us so.  Every form does the
+// same operations on each value.
 constexpr int kEdgeThreads = 128;
-template <int FLUX, int C>
-__device__ __forceinline__ void edge_flux_f64(const ArenaPtrs<F64> &A, const MeshConst &mc,
-                                              const R4<F64> *P, int e, double *face, F64T<C> f[4],
-                                              int &err) {
-  using T = F64T<C>;
-  const int2 nn = A.be_nodes[e];
-  const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
-  const double dx = c2.x - c1.x, dy = c2.y - c1.y;
+template <int C>
+constexpr int kEdgeItem = C == 2 ? kEdgeThreads / 4 : kEdgeThreads;
+
+template <int C>
+__device__ __forceinline__ void edge_recon_f64(const ArenaPtrs<F64> &A, const MeshConst &mc,
+                                               const R4<F64> *P, int2 nn, double dx, double dy,
+                                               int q, double *face, int stride) {
   const double *s1 = reinterpret_cast<const double *>(P + nn.x);
   const double *s2 = reinterpret_cast<const double *>(P + nn.y);
   const double *g1 = reinterpret_cast<const double *>(A.grad + nn.x);
   const double *g2 = reinterpret_cast<const double *>(A.grad + nn.y);
-#pragma unroll 1
-  for (int q = 0; q < 4; q++) {
-    double pl, pr;
-    recon1_f64<C>(s1[q], s2[q], g1[q], g1[4 + q], g2[q], g2[4 + q], dx, dy, mc.ilimit,
-                  mc.albada11, mc.albada12, mc.albada21, mc.albada22, mc.epsilon, pl, pr);
-    face[q * kEdgeThreads] = pl;
-    face[(4 + q) * kEdgeThreads] = pr;
-  }
+  double pl, pr;
+  recon1_f64<C>(s1[q], s2[q], g1[q], g1[4 + q], g2[q], g2[4 + q], dx, dy, mc.ilimit, mc.albada11,
+                mc.albada12, mc.albada21, mc.albada22, mc.epsilon, pl, pr);
+  face[q * stride] = pl;
+  face[(4 + q) * stride] = pr;
+}
+
+template <int FLUX, int C>
+__device__ __forceinline__ R4<F64> edge_riemann_f64(const ArenaPtrs<F64> &A, const MeshConst &mc,
+                                                    int e, double *face, int stride, int &err) {
+  using T = F64T<C>;
   const D4 csl = A.be_csl[e];
   const FluxConst<T> fc = flux_const<T>(mc);
+  T f[4];
+  bool ok;
   if constexpr (FLUX == 1) {
-    if (!roe_flux_f64<C>(face, kEdgeThreads, csl.x, csl.y, csl.z, fc.gamma, fc.gamma1, f)) err = 1;
-    return;
-  }
-  T pl[4], pr[4];
+    ok = roe_flux_f64<C>(face, stride, csl.x, csl.y, csl.z, fc.gamma, fc.gamma1, f);
+  } else {
+    T pl[4], pr[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    pl[q] = face[q * kEdgeThreads];
-    pr[q] = face[(4 + q) * kEdgeThreads];
+    for (int q = 0; q < 4; q++) {
+      pl[q] = face[q * stride];
+      pr[q] = face[(4 + q) * stride];
+    }
+    ok = riemann<T, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f);
   }
-  if (!riemann<T, FLUX>(fc, csl.x, csl.y, csl.z, pl, pr, f)) err = 1;
+  if (!ok) err = 1;
+  R4<F64> o;
+  o.x = f[0].v;
+  o.y = f[1].v;
+  o.z = f[2].v;
+  o.w = f[3].v;
+  return o;
 }
 
 // One boundary edge: its contributions to n1 and n2.
@@ -1362,7 +1385,7 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // entry of the block owning it), and of every boundary edge into bflux.  The
 // FP64 pipe bounds it: 2 lanes per SM and clock against ~430 operations per
 // edge, so nothing may be computed twice and no SM may idle.  One work item
-// is kEdgeThreads owned entries of a block (the last item of a block: its
+// is kEdgeItem<C> owned entries of a block (the last item of a block: its
 // boundary edges), many items per SM.  One kernel over whole blocks computed
 // cut edges in both blocks (+10%) and left most SMs idle in its last wave:
 // 1365 us for 1024 x 384, Roe; 1000 us here on the FP64 pipe alone (446
@@ -1375,10 +1398,15 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // SM: 442 us; the rule is in update_work.  HLLC on 768 x 256: 1064 -> 560 us,
 // its pow still on the FP64 pipe.
 template <typename R, int FLUX, int C>
-__global__ void __launch_bounds__(kEdgeThreads, C ? FVM_EFLUX_CALLB : FVM_EFLUX_MINB)
+__global__ void __launch_bounds__(kEdgeThreads, C == 2   ? FVM_EFLUX_FEWB
+                                                : C == 1 ? FVM_EFLUX_CALLB
+                                                         : FVM_EFLUX_MINB)
     k_eflux(ArenaPtrs<R> A, int stage, int routine, int items) {
   static_assert(sizeof(R) == 8, "the FP64 pass");
-  __shared__ double s_face[(FLUX == 1 ? 12 : 8) * kEdgeThreads];
+  constexpr int stride = kEdgeItem<C>;
+  __shared__ double s_face[(FLUX == 1 ? 12 : 8) * stride];
+  const int lane = threadIdx.x % stride;
+  double *face = s_face + lane;
   int w0, nwork;
   work_range(A, w0, nwork);
   for (int i = w0 * items + blockIdx.x; i < nwork * items; i += gridDim.x) {
@@ -1393,17 +1421,30 @@ __global__ void __launch_bounds__(kEdgeThreads, C ? FVM_EFLUX_CALLB : FVM_EFLUX_
         boundary_row(A, mc, ctl, bi.b0 + k / 4, P, k & 3);
       continue;
     }
-    const int k = c * kEdgeThreads + threadIdx.x;
-    if (k >= A.blk_neo[bi.part]) continue;
+    const int neo = A.blk_neo[bi.part];
+    if (c * stride >= neo) continue;
+    const bool have = c * stride + lane < neo;
+    const int e = bi.e0 + c * stride + lane;
+    int2 nn = make_int2(0, 0);
+    double dx = 0.0, dy = 0.0;
+    if (have) {
+      nn = A.be_nodes[e];
+      const double2 c1 = A.coord[nn.x], c2 = A.coord[nn.y];
+      dx = c2.x - c1.x;
+      dy = c2.y - c1.y;
+    }
+    if constexpr (kEdgeItem<C> < kEdgeThreads) {
+      __syncthreads();   // the CTA's last item has been read
+      if (have) edge_recon_f64<C>(A, mc, P, nn, dx, dy, threadIdx.x / stride, face, stride);
+      __syncthreads();
+      if (!have || threadIdx.x >= stride) continue;
+    } else {
+      if (!have) continue;
+#pragma unroll 1
+      for (int q = 0; q < 4; q++) edge_recon_f64<C>(A, mc, P, nn, dx, dy, q, face, stride);
+    }
     int err = 0;
-    F64T<C> f[4];
-    edge_flux_f64<FLUX, C>(A, mc, P, bi.e0 + k, s_face + threadIdx.x, f, err);
-    R4<R> o;
-    o.x = f[0].v;
-    o.y = f[1].v;
-    o.z = f[2].v;
-    o.w = f[3].v;
-    A.eflux[bi.e0 + k] = o;
+    A.eflux[e] = edge_riemann_f64<FLUX, C>(A, mc, e, face, stride, err);
     if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
   }
 }

@@ -56,16 +56,21 @@ inline void launch_flux_code(const ArenaPtrs<R> &A, const LaunchCfg &c, int stag
     k_flux<KT<R>, F><<<fit_grid(c, k_flux<KT<R>, F>, sm, kFluxThreads), kFluxThreads, sm, c.stream>>>(
         kptrs(A), stage, mode, irk, routine);
   } else {
-    // a block's owned entries in items of kEdgeThreads, and its boundary edges
-    const int items = (c.max_slots + kEdgeThreads - 1) / kEdgeThreads + 1;
+    // a block's owned entries in items, and its boundary edges
+    const int per = c.edge_form == 2 ? kEdgeItem<2> : kEdgeThreads;
+    const int items = (c.max_slots + per - 1) / per + 1;
     LaunchCfg ce = c;
     ce.grid = c.grid > INT_MAX / items ? INT_MAX : c.grid * items;
-    if (c.edge_calls)
-      k_eflux<KT<R>, F, 1><<<fit_grid(ce, k_eflux<KT<R>, F, 1>, 0, kEdgeThreads), kEdgeThreads, 0,
-                             c.stream>>>(kptrs(A), stage, routine, items);
+#define FVM_EFLUX(C)                                                                       \
+  k_eflux<KT<R>, F, C><<<fit_grid(ce, k_eflux<KT<R>, F, C>, 0, kEdgeThreads), kEdgeThreads, 0, \
+                         c.stream>>>(kptrs(A), stage, routine, items)
+    if (c.edge_form == 2)
+      FVM_EFLUX(2);
+    else if (c.edge_form == 1)
+      FVM_EFLUX(1);
     else
-      k_eflux<KT<R>, F, 0><<<fit_grid(ce, k_eflux<KT<R>, F, 0>, 0, kEdgeThreads), kEdgeThreads, 0,
-                             c.stream>>>(kptrs(A), stage, routine, items);
+      FVM_EFLUX(0);
+#undef FVM_EFLUX
     k_egather<KT<R>><<<fit_grid(c, k_egather<KT<R>>, 0), kBlockVerts, 0, c.stream>>>(kptrs(A), stage, mode, irk,
                                                                              routine);
   }

@@ -29,7 +29,7 @@ struct LaunchCfg {
   bool any_inviscid; // an inviscid mesh is resident
   int pipe_groups;   // consumer groups of a pipelined kernel's CTA (1 or 2)
   int pipe_stages;   // stages of its ring (0: as many as fit, at most kPipeMaxStages)
-  bool edge_calls;   // FP64 edge pass with called operations (many edges; see update_work)
+  int edge_form;     // FP64 edge pass: k_eflux's C, by the edges at work (see update_work)
   bool std_const;    // every resident mesh has math.f's constants (FP32 flux pass folds them)
   cudaStream_t stream;
 };
