@@ -503,6 +503,125 @@ __device__ __forceinline__ void hllc_flux(R ct, R st, R length, const R pl4[4], 
   flux[3] = f3 * length;
 }
 
+// FP64: hllc_flux in three parts, its values in shared memory as roe_flux_f64's
+// (face: after the first part rho, u_n, u_t, p of each side, then a_l, a_r,
+// p*, u*), so that the caller can have the pow of a CTA's rarefaction fans done
+// by all of its threads in between.  The operations and their order are
+// hllc_flux's.
+//
+// First part: true if the star state is the two-rarefaction one, which
+// hllc_rare_f64 then forms from pow(pl, z), pow(pr, z), pow(pl / pr, z).
+template <int C>
+__device__ __forceinline__ bool hllc_star_f64(volatile double *face, int stride, F64T<C> ct,
+                                              F64T<C> st, F64T<C> gamma) {
+  using F64 = F64T<C>;
+  auto in = [&](int q) { return F64(face[q * stride]); };
+  auto put = [&](int q, F64 x) { face[q * stride] = x.v; };
+#pragma unroll 1
+  for (int k = 0; k < 2; k++) {
+    const F64 u = in(4 * k + 1), v = in(4 * k + 2);
+    put(4 * k + 1, u * ct + v * st);
+    put(4 * k + 2, -u * st + v * ct);
+    put(8 + k, msqrt(mdiv(gamma * in(4 * k + 3), in(4 * k))));
+  }
+  const F64 pl = in(3), pr = in(7), ul = in(1), ur = in(5);
+  const F64 rbar = half(in(0) + in(4));
+  const F64 abar = half(in(8) + in(9));
+  const F64 Ppv = half(pl + pr - (ur - ul) * rbar * abar);
+  const F64 Upv = half(ul + ur - mdiv(pr - pl, rbar * abar));
+  F64 prmax = pr, prmin = pl;
+  if (pl > pr) {
+    prmax = pl;
+    prmin = pr;
+  }
+  const F64 Q = mdiv(prmax, prmin);
+  if (Q < F64(2.0) && prmin < Ppv && Ppv < prmax) {
+    put(10, Ppv);
+    put(11, Upv);
+    return false;
+  }
+  if (Ppv < prmin) return true;
+  const F64 po = dmax1(F64(0.0), Ppv);
+  F64 g[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const F64 M = F64(2.0) / (gamma + F64(1.0)) / in(4 * k);
+    const F64 N = (gamma - F64(1.0)) * in(4 * k + 3) / (gamma + F64(1.0));
+    g[k] = msqrt(M / (po + N));
+  }
+  const F64 a1 = g[0] * pl + g[1] * pr - (ur - ul);
+  const F64 pstar = a1 / (g[0] + g[1]);
+  put(10, pstar);
+  put(11, half(ul + ur + (pstar - pr) * g[1] - (pstar - pl) * g[0]));
+  return false;
+}
+
+// The two-rarefaction u*, and the base of the power 1 / z that is p*.
+template <int C>
+__device__ __forceinline__ double hllc_rare_f64(volatile double *face, int stride, F64T<C> gamma,
+                                                double pzl, double pzr, double pzlr) {
+  using F64 = F64T<C>;
+  auto in = [&](int q) { return F64(face[q * stride]); };
+  const F64 ul = in(1), ur = in(5), al = in(8), ar = in(9), Plr = pzlr;
+  const F64 a1 = al + ar - F64(0.5) * (gamma - F64(1.0)) * (ur - ul);
+  const F64 a2 = al / F64(pzl) + ar / F64(pzr);
+  const F64 b1 = Plr * ul / al + ur / ar + F64(2.0) * (Plr - F64(1.0)) / (gamma - F64(1.0));
+  const F64 b2 = Plr / al + F64(1.0) / ar;
+  face[11 * stride] = (b1 / b2).v;
+  return (a1 / a2).v;
+}
+
+// The flux from the star state.
+template <int C>
+__device__ __forceinline__ void hllc_flux_f64(volatile double *face, int stride, F64T<C> ct,
+                                              F64T<C> st, F64T<C> length, F64T<C> gamma,
+                                              F64T<C> GAMMA1, int rotate_back, F64T<C> flux[4]) {
+  using F64 = F64T<C>;
+  auto in = [&](int q) { return F64(face[q * stride]); };
+  const F64 pstar = in(10), Ss = in(11);
+  F64 S[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const F64 pk = in(4 * k + 3);
+    F64 q = F64(1.0);
+    if (!(pstar <= pk))
+      q = msqrt(F64(1.0) +
+                mdiv(F64(0.5) * (gamma + F64(1.0)) * (mdiv(pstar, pk) - F64(1.0)), gamma));
+    const F64 aq = in(8 + k) * q;
+    S[k] = k ? in(5) + aq : in(1) - aq;
+  }
+  const F64 Sl = S[0], Sr = S[1];
+  const bool c1 = F64(0.0) <= Sl;
+  const bool c2 = !c1 && Sl <= F64(0.0) && F64(0.0) <= Ss;
+  const bool c3 = !c1 && !c2 && Ss <= F64(0.0) && F64(0.0) <= Sr;
+  const bool left = c1 || c2, star = c2 || c3;
+  const int o = left ? 0 : 4;
+  const F64 rk = in(o), uk = in(o + 1), vk = in(o + 2), pk = in(o + 3), Sk = left ? Sl : Sr;
+  const F64 Ek = mdiv(pk, GAMMA1) + half(rk) * (sq(uk) + sq(vk));
+  F64 f0 = rk * uk, f1 = pk + rk * sq(uk), f2 = rk * uk * vk, f3 = (Ek + pk) * uk;
+  if (star) {
+    const F64 fact = mdiv(rk * (Sk - uk), Sk - Ss);
+    const F64 du0 = fact - rk;
+    const F64 du1 = fact * Ss - rk * uk;
+    const F64 du2 = fact * vk - rk * vk;
+    const F64 t1 = mdiv(Ek, rk) + (Ss - uk) * (Ss + mdiv(mdiv(pk, rk), Sk - uk));
+    const F64 du3 = fact * t1 - Ek;
+    f0 = f0 + Sk * du0;
+    f1 = f1 + Sk * du1;
+    f2 = f2 + Sk * du2;
+    f3 = f3 + Sk * du3;
+  }
+  if (rotate_back) {
+    const F64 fn = f1, ft = f2;
+    f1 = ct * fn - st * ft;
+    f2 = st * fn + ct * ft;
+  }
+  flux[0] = f0 * length;
+  flux[1] = f1 * length;
+  flux[2] = f2 * length;
+  flux[3] = f3 * length;
+}
+
 // ------------------------------------------------------ farfield_flux.f
 // The state outside a farfield edge: freestream, or with the point-vortex
 // correction (farfield_flux.f:28-44, evaluated in FP64).

@@ -1169,14 +1169,17 @@ __device__ __forceinline__ void edge_recon_f64(const ArenaPtrs<F64> &A, const Me
 
 template <int FLUX, int C>
 __device__ __forceinline__ R4<F64> edge_riemann_f64(const ArenaPtrs<F64> &A, const MeshConst &mc,
-                                                    int e, double *face, int stride, int &err) {
+                                                    const D4 &csl, double *face, int stride,
+                                                    int &err) {
   using T = F64T<C>;
-  const D4 csl = A.be_csl[e];
   const FluxConst<T> fc = flux_const<T>(mc);
   T f[4];
   bool ok;
   if constexpr (FLUX == 1) {
     ok = roe_flux_f64<C>(face, stride, csl.x, csl.y, csl.z, fc.gamma, fc.gamma1, f);
+  } else if constexpr (FLUX == 3) {
+    hllc_flux_f64<C>(face, stride, csl.x, csl.y, csl.z, fc.gamma, fc.gamma1, fc.rotate_back, f);
+    ok = true;
   } else {
     T pl[4], pr[4];
 #pragma unroll
@@ -1193,6 +1196,53 @@ __device__ __forceinline__ R4<F64> edge_riemann_f64(const ArenaPtrs<F64> &A, con
   o.z = f[2].v;
   o.w = f[3].v;
   return o;
+}
+
+// HLLC: the edges of a CTA whose star state is a two-rarefaction one (a
+// minority, but in nearly every warp) put the bases of their four pow into
+// shared memory, and all threads of the CTA take one each: pow is ~100
+// operations of the FP64 pipe, which a branch would pass four times per warp
+// (768 x 256, turbulent: 560 -> 390 us).
+// Called by every thread of the CTA (barriers); `mine`: this thread has an edge.
+template <int C>
+__device__ __forceinline__ void edge_hllc_star(const MeshConst &mc, const D4 &csl, bool mine,
+                                               double *face, int stride, double *s_pow,
+                                               int *s_n) {
+  using T = F64T<C>;
+  const T gamma = mc.gamma;
+  bool rare = false;
+  if (mine) rare = hllc_star_f64<C>(face, stride, csl.x, csl.y, gamma);
+  const uint32_t warp = __ballot_sync(0xffffffffu, rare);
+  int k = 0;
+  if (warp) {
+    if ((threadIdx.x & 31) == 0) k = atomicAdd(s_n, __popc(warp));
+    k = __shfl_sync(0xffffffffu, k, 0) + __popc(warp & ((1u << (threadIdx.x & 31)) - 1));
+  }
+  if (rare) {
+    const T pl = face[3 * stride], pr = face[7 * stride];
+    s_pow[3 * k] = pl.v;
+    s_pow[3 * k + 1] = pr.v;
+    s_pow[3 * k + 2] = (pl / pr).v;
+  }
+  const int n = __syncthreads_count(rare);
+  if (n == 0) return;
+  const T z = T(0.5) * (gamma - T(1.0)) / gamma;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < 3 * n; t += kEdgeThreads) s_pow[t] = pow(s_pow[t], z.v);
+  __syncthreads();
+  // (the bases of p* in rows of their own: the next item's bases may be
+  // written while the last threads still read these)
+  double *s_star = s_pow + 3 * stride;
+  if (threadIdx.x == 0) *s_n = 0;
+  if (rare)
+    s_star[k] = hllc_rare_f64<C>(face, stride, gamma, s_pow[3 * k], s_pow[3 * k + 1],
+                                 s_pow[3 * k + 2]);
+  __syncthreads();
+  const T z1 = T(1.0) / z;
+#pragma unroll 1
+  for (int t = threadIdx.x; t < n; t += kEdgeThreads) s_star[t] = pow(s_star[t], z1.v);
+  __syncthreads();
+  if (rare) face[10 * stride] = s_star[k];
 }
 
 // One boundary edge: its contributions to n1 and n2.
@@ -1396,7 +1446,7 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // operations instead of inlining them, and few live values (the reconstructed
 // states and the central flux wait in shared memory) let seven CTAs share an
 // SM: 442 us; the rule is in update_work.  HLLC on 768 x 256: 1064 -> 560 us,
-// its pow still on the FP64 pipe.
+// 390 us since its pow are shared out (edge_hllc_star).
 template <typename R, int FLUX, int C>
 __global__ void __launch_bounds__(kEdgeThreads, C == 2   ? FVM_EFLUX_FEWB
                                                 : C == 1 ? FVM_EFLUX_CALLB
@@ -1404,9 +1454,15 @@ __global__ void __launch_bounds__(kEdgeThreads, C == 2   ? FVM_EFLUX_FEWB
     k_eflux(ArenaPtrs<R> A, int stage, int routine, int items) {
   static_assert(sizeof(R) == 8, "the FP64 pass");
   constexpr int stride = kEdgeItem<C>;
-  __shared__ double s_face[(FLUX == 1 ? 12 : 8) * stride];
+  // rows of face, and HLLC's bases and powers
+  __shared__ double s_face[(FLUX == 3 ? 16 : FLUX == 1 ? 12 : 8) * stride];
+  __shared__ int s_n;
   const int lane = threadIdx.x % stride;
   double *face = s_face + lane;
+  if (FLUX == 3) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+  }
   int w0, nwork;
   work_range(A, w0, nwork);
   for (int i = w0 * items + blockIdx.x; i < nwork * items; i += gridDim.x) {
@@ -1433,18 +1489,25 @@ __global__ void __launch_bounds__(kEdgeThreads, C == 2   ? FVM_EFLUX_FEWB
       dx = c2.x - c1.x;
       dy = c2.y - c1.y;
     }
+    bool mine = have;
     if constexpr (kEdgeItem<C> < kEdgeThreads) {
       __syncthreads();   // the CTA's last item has been read
       if (have) edge_recon_f64<C>(A, mc, P, nn, dx, dy, threadIdx.x / stride, face, stride);
       __syncthreads();
-      if (!have || threadIdx.x >= stride) continue;
-    } else {
-      if (!have) continue;
+      mine = have && threadIdx.x < stride;
+    } else if (have) {
 #pragma unroll 1
       for (int q = 0; q < 4; q++) edge_recon_f64<C>(A, mc, P, nn, dx, dy, q, face, stride);
     }
+    if (FLUX != 3 && !mine) continue;
+    D4 csl;
+    if (mine) csl = A.be_csl[e];
+    if constexpr (FLUX == 3) {
+      edge_hllc_star<C>(mc, csl, mine, face, stride, s_face + 12 * stride, &s_n);
+      if (!mine) continue;
+    }
     int err = 0;
-    A.eflux[e] = edge_riemann_f64<FLUX, C>(A, mc, e, face, stride, err);
+    A.eflux[e] = edge_riemann_f64<FLUX, C>(A, mc, csl, face, stride, err);
     if (err) atomicCAS(&ctl.err, 0, 4 /* FVM_ERR_ROE_SONIC */);
   }
 }
