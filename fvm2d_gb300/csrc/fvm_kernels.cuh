@@ -32,6 +32,9 @@
 #ifndef FVM_GRAD_MINB64
 #define FVM_GRAD_MINB64 4   // the same of the FP64 one for inviscid meshes (3, 5: the same)
 #endif
+#ifndef FVM_GRAD_MINBV64
+#define FVM_GRAD_MINBV64 3  // the same with viscous ones (2: 14-25% slower, 4: the same)
+#endif
 #ifndef FVM_GRADV_MINB32
 #define FVM_GRADV_MINB32 4  // the same for its per-vertex form
 #endif
@@ -391,11 +394,14 @@ __device__ __forceinline__ void grad_vertex_sums(const uint16_t *vtl, int j0, in
   }
 }
 
-// FP64, inviscid meshes: the sums of the four variables one after another (the
-// integer products make long code), the triangle sums as rows of max_tri in
-// shared memory, s[2 q] and s[2 q + 1] of variable q (random 64-byte records
-// conflict in the banks).  Few live values: four CTAs share an SM instead of
-// two; 136 -> 107 us on 1024 x 384.
+// FP64: the sums of the four variables one after another (the integer products
+// make long code), the triangle sums as rows of max_tri in shared memory, s[2 q]
+// and s[2 q + 1] of variable q (random 64-byte records conflict in the banks).
+// Few live values: four CTAs share an SM instead of two; 1024 x 384: 136 -> 107
+// us.  Viscous meshes' terms follow in a second round over the triangles and
+// vertices, in the same rows: 72 bytes per triangle instead of 136, three CTAs;
+// 512 x 192 laminar 86 -> 72 us, 768 x 256 turbulent 168 -> 160 (called
+// operations: 85 and 182).
 template <typename R>
 __device__ __forceinline__ void tri_sums_rows(const ArenaPtrs<R> &A, const R4<R> *P, int entry,
                                               int k, R *s, int max_tri) {
@@ -412,13 +418,39 @@ __device__ __forceinline__ void tri_sums_rows(const ArenaPtrs<R> &A, const R4<R>
   }
 }
 
-// VISC: viscous meshes may be among the blocks
-template <typename R, bool VISC>
+// The viscous terms of triangle k into rows 0..8 (the sums' rows, which its
+// vertices have been given): row 3 pos + c is component c at position pos.
+template <typename R>
+__device__ __forceinline__ void tri_visc_rows(const ArenaPtrs<R> &A, const MeshConst &mc, int nbuf,
+                                              const R4<R> *P, int entry, int k, R *s,
+                                              int max_tri) {
+  const int4 t = A.bt_nodes[entry];
+  R dbxx[3], dbyy[3];
+  tri_geom<R>(A, t, entry, dbxx, dbyy);
+  TriSmem<R> ts;
+  ts.dxt[1] = s[2 * max_tri + k];
+  ts.dyt[1] = s[3 * max_tri + k];
+  ts.dxt[2] = s[4 * max_tri + k];
+  ts.dyt[2] = s[5 * max_tri + k];
+  const TriVisc<R> tv = tri_visc<R>(A, mc, nbuf, t, tri_areat<R>(A, t, entry), P[t.x], P[t.y],
+                                    P[t.z], dbxx, dbyy, ts);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    R o[3];
+    tri_visc_term<R>(tv, dbxx[j], dbyy[j], o);
+#pragma unroll
+    for (int c = 0; c < 3; c++) s[(3 * j + c) * max_tri + k] = o[c];
+  }
+}
+
+// FORM 0: sums and viscous terms of a triangle as records, one round; FP64 also
+// as rows: 1 inviscid meshes only, 2 viscous ones too, in two rounds.
+template <typename R, int FORM>
 __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32
-                                               : VISC         ? 2
-                                                              : FVM_GRAD_MINB64)
-    k_grad(ArenaPtrs<R> A, int stage, int do_dt,
-                                                      int routine, int max_tri, int skip_inviscid) {
+                                               : FORM == 0    ? 2
+                                               : FORM == 1    ? FVM_GRAD_MINB64
+                                                              : FVM_GRAD_MINBV64)
+    k_grad(ArenaPtrs<R> A, int stage, int do_dt, int routine, int max_tri, int skip_inviscid) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TriSmem<R> *s_tri = reinterpret_cast<TriSmem<R> *>(smem_raw);
   R *s_vis = reinterpret_cast<R *>(s_tri + max_tri);   // [max_tri][3 pos][3 comp]
@@ -430,8 +462,7 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32
     if (!routine && !ctl.active) continue;
     const MeshConst &mc = A.mc[bi.mesh];
     if (skip_inviscid && mc.iflow == 1) continue;   // the stencil pass's meshes
-    const bool visc = VISC && mc.iflow != 1;
-    constexpr bool rows = sizeof(R) == 8 && !VISC;
+    const bool visc = FORM != 1 && mc.iflow != 1;
     const R4<R> *P = A.st[cur_buf(ctl.phase, stage)];
     if (threadIdx.x == 0) {
       const BlockInfo *nb = next_block(A, w, nwork);
@@ -445,34 +476,17 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32
         prefetch_l2(sizeof(R) == 4 ? (const void *)(A.ais32 + n.v0) : (const void *)(A.ais + n.v0), sizeof(R) * n.nv);
       }
     }
-    // phase 1: one thread per triangle touching the block
-    for (int k = threadIdx.x; k < bi.nt; k += blockDim.x) {
-      if constexpr (rows) {
-        tri_sums_rows<R>(A, P, bi.t0 + k, k, reinterpret_cast<R *>(smem_raw), max_tri);
-        continue;
-      }
-      const int4 t = A.bt_nodes[bi.t0 + k];
-      const R4<R> p1 = P[t.x], p2 = P[t.y], p3 = P[t.z];
-      R dbxx[3], dbyy[3];
-      tri_geom<R>(A, t, bi.t0 + k, dbxx, dbyy);
-      TriSmem<R> ts;
-      tri_sums<R>(p1, p2, p3, dbxx, dbyy, ts);
-      s_tri[k] = ts;
-      if (visc) {
-        const TriVisc<R> tv = tri_visc<R>(A, mc, ctl.nphase, t, tri_areat<R>(A, t, bi.t0 + k), p1, p2, p3, dbxx, dbyy, ts);
-        R *sv = s_vis + 9 * k;
-#pragma unroll
-        for (int j = 0; j < 3; j++) tri_visc_term<R>(tv, dbxx[j], dbyy[j], sv + 3 * j);
-      }
-    }
-    __syncthreads();
-    // phase 2: one thread per vertex, triangles in original order
-    if (threadIdx.x < bi.nv) {
+    if constexpr (FORM != 0) {
+      R *s = reinterpret_cast<R *>(smem_raw);
       const int v = bi.v0 + threadIdx.x;
-      R qx[4], qy[4], rv[3];
-      const int2 jr = A.vt_rng[v];
-      if constexpr (rows) {
-        const R *s = reinterpret_cast<const R *>(smem_raw);
+      const bool mine = threadIdx.x < bi.nv;
+      int2 jr = make_int2(0, 0);
+      if (mine) jr = A.vt_rng[v];
+      for (int k = threadIdx.x; k < bi.nt; k += blockDim.x)
+        tri_sums_rows<R>(A, P, bi.t0 + k, k, s, max_tri);
+      __syncthreads();
+      if (mine) {
+        R qx[4], qy[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) qx[q] = qy[q] = R(0);
         for (int j = jr.x; j < jr.y; j++) {
@@ -483,31 +497,84 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32
             qy[q] = qy[q] + e[(2 * q + 1) * max_tri];
           }
         }
-      } else {
+        const R ais = v_ais(A, v);
+        Grad<R> g;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          g.qx[q] = qx[q] * ais;
+          g.qy[q] = qy[q] * ais;
+        }
+        A.grad[v] = g;
+        if (!visc && do_dt) A.dt[v] = time_step<R>(mc, P[v], R(0), v_drmin(A, v));
+      }
+      __syncthreads();
+      if (!visc) continue;
+      for (int k = threadIdx.x; k < bi.nt; k += blockDim.x)
+        tri_visc_rows<R>(A, mc, ctl.nphase, P, bi.t0 + k, k, s, max_tri);
+      __syncthreads();
+      if (mine) {
+        R rv[3] = {R(0), R(0), R(0)};
+        for (int j = jr.x; j < jr.y; j++) {
+          const int u = A.vt_list[j];
+          const R *e = s + 3 * (u >> kTriPosShift) * max_tri + (u & 0x3fff);
+#pragma unroll
+          for (int c = 0; c < 3; c++) rv[c] = rv[c] + e[c * max_tri];
+        }
+        R4<R> o;
+        o.x = R(0);
+        o.y = rv[0];
+        o.z = rv[1];
+        o.w = rv[2];
+        A.resv[v] = o;
+      }
+      __syncthreads();
+    } else {
+      // phase 1: one thread per triangle touching the block
+      for (int k = threadIdx.x; k < bi.nt; k += blockDim.x) {
+        const int4 t = A.bt_nodes[bi.t0 + k];
+        const R4<R> p1 = P[t.x], p2 = P[t.y], p3 = P[t.z];
+        R dbxx[3], dbyy[3];
+        tri_geom<R>(A, t, bi.t0 + k, dbxx, dbyy);
+        TriSmem<R> ts;
+        tri_sums<R>(p1, p2, p3, dbxx, dbyy, ts);
+        s_tri[k] = ts;
+        if (visc) {
+          const TriVisc<R> tv = tri_visc<R>(A, mc, ctl.nphase, t, tri_areat<R>(A, t, bi.t0 + k), p1, p2, p3, dbxx, dbyy, ts);
+          R *sv = s_vis + 9 * k;
+#pragma unroll
+          for (int j = 0; j < 3; j++) tri_visc_term<R>(tv, dbxx[j], dbyy[j], sv + 3 * j);
+        }
+      }
+      __syncthreads();
+      // phase 2: one thread per vertex, triangles in original order
+      if (threadIdx.x < bi.nv) {
+        const int v = bi.v0 + threadIdx.x;
+        R qx[4], qy[4], rv[3];
+        const int2 jr = A.vt_rng[v];
         // (FP32: one triangle at a time, the 48 registers of five CTAs per SM)
         grad_vertex_sums<R, sizeof(R) == 8 ? 2 : 1>(A.vt_list, jr.x, jr.y, s_tri,
                                                     visc ? s_vis : nullptr, qx, qy, rv);
-      }
-      const R ais = v_ais(A, v);
-      Grad<R> g;
+        const R ais = v_ais(A, v);
+        Grad<R> g;
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        g.qx[q] = qx[q] * ais;
-        g.qy[q] = qy[q] * ais;
+        for (int q = 0; q < 4; q++) {
+          g.qx[q] = qx[q] * ais;
+          g.qy[q] = qy[q] * ais;
+        }
+        A.grad[v] = g;
+        if (visc) {
+          R4<R> r;
+          r.x = R(0);
+          r.y = rv[0];
+          r.z = rv[1];
+          r.w = rv[2];
+          A.resv[v] = r;
+        } else if (do_dt) {
+          A.dt[v] = time_step<R>(mc, P[v], R(0), v_drmin(A, v));
+        }
       }
-      A.grad[v] = g;
-      if (visc) {
-        R4<R> r;
-        r.x = R(0);
-        r.y = rv[0];
-        r.z = rv[1];
-        r.w = rv[2];
-        A.resv[v] = r;
-      } else if (do_dt) {
-        A.dt[v] = time_step<R>(mc, P[v], R(0), v_drmin(A, v));
-      }
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 

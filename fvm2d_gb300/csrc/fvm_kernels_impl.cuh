@@ -46,6 +46,46 @@ inline int fit_grid(const LaunchCfg &c, K kern, size_t smem, int threads = kBloc
   return g < c.grid ? g : c.grid;
 }
 
+// FP64 gradient: rows for inviscid meshes, and for viscous ones where the
+// records (136 bytes per triangle) would leave an SM two CTAs, that is blocks of
+// 256 vertices; blocks of 64 or 128 keep the one round.  us per iteration,
+// records / rows: 512 x 192 laminar 838 / 798, 768 x 256 turbulent 2124 / 2092;
+// 300 x 90 laminar (128 vertices) 370 / 377, 160 x 48 turbulent 270 / 276.
+// sm: the records' bytes, never less than the rows'.
+template <typename R>
+inline cudaError_t launch_grad_f64(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int do_dt,
+                                   int routine, size_t sm) {
+  if constexpr (sizeof(R) == 8) {
+    const int form = !c.viscous ? 1 : sm > kMaxSmem / 3 ? 2 : 0;
+    if (form) sm = size_t(c.max_tri) * (form == 2 ? 9 : 8) * sizeof(R);
+#define FVM_GRAD64(F)                                                                      \
+  k_grad<KT<R>, F><<<fit_grid(c, k_grad<KT<R>, F>, sm), kBlockVerts, sm, c.stream>>>(      \
+      kptrs(A), stage, do_dt, routine, c.max_tri, 0)
+    if (form == 1)
+      FVM_GRAD64(1);
+    else if (form == 2)
+      FVM_GRAD64(2);
+    else
+      FVM_GRAD64(0);
+#undef FVM_GRAD64
+  }
+  return cudaGetLastError();
+}
+template <typename R>
+inline cudaError_t grad_attributes(size_t sm) {
+  cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>, 0>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if constexpr (sizeof(R) == 8) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_grad<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sm);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_grad<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sm);
+  }
+  return e;
+}
+
 // The flux pass for template code F (Riemann solver | kFluxStd).  FP32: one
 // kernel; FP64: every edge once, then the gather.
 template <typename R, int F>
@@ -182,13 +222,9 @@ inline cudaError_t flux_attributes(size_t f) {
           kptrs(A), stage, do_dt, routine, c.max_tri, c.max_halo, c.viscous ? 1 : 0, skip);       \
       return cudaGetLastError();                                                           \
     }                                                                                      \
-    /* FP32: viscous meshes alone reach this form */                                       \
-    if (sizeof(R) == 4 || c.viscous)                                                       \
-      k_grad<KT<R>, true><<<fit_grid(c, k_grad<KT<R>, true>, sm), kBlockVerts, sm, c.stream>>>( \
-          kptrs(A), stage, do_dt, routine, c.max_tri, skip);                               \
-    else                                                                                   \
-      k_grad<KT<R>, (sizeof(R) == 4)><<<fit_grid(c, k_grad<KT<R>, (sizeof(R) == 4)>, sm), kBlockVerts, sm, c.stream>>>( \
-          kptrs(A), stage, do_dt, routine, c.max_tri, skip);                               \
+    if constexpr (sizeof(R) == 8) return launch_grad_f64(A, c, stage, do_dt, routine, sm);  \
+    k_grad<KT<R>, 0><<<fit_grid(c, k_grad<KT<R>, 0>, sm), kBlockVerts, sm, c.stream>>>(     \
+        kptrs(A), stage, do_dt, routine, c.max_tri, skip);                                 \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_flux(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage, int mode,   \
@@ -276,11 +312,7 @@ inline cudaError_t flux_attributes(size_t f) {
       if (k == 3) e2 = cudaFuncSetAttribute(k_step<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
       if (e2 != cudaSuccess) return e2;                                                    \
     }                                                                                      \
-    cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>, true>,                              \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g); \
-    if (e == cudaSuccess)                                                                  \
-      e = cudaFuncSetAttribute(k_grad<KT<R>, (sizeof(R) == 4)>,                      \
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g);       \
+    cudaError_t e = grad_attributes<R>(g);                                                 \
     if (e == cudaSuccess) e = flux_attributes<R>(f);                                       \
     if (e == cudaSuccess)                                                                  \
       e = cudaFuncSetAttribute(k_sa<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s); \
