@@ -352,14 +352,39 @@ __device__ __forceinline__ void tri_visc_term(const TriVisc<R> &tv, R dbx, R dby
   out[2] = (tv.efx * dbx + tv.efy * dby) * tv.areat;
 }
 
+// FP32 triangle sums in shared memory, the record's two 16-byte halves swapped
+// where bit 2 of the slot is set: neighbouring threads read slots one or two
+// apart, whose like halves would share a quarter or half of the banks (60% of
+// the gradient's shared-memory wavefronts were conflicts; 4 x 768x256 turbulent
+// 0.072 -> 0.064 ms per stage, the 24-mesh mix 0.132 -> 0.122, and 0.399 ->
+// 0.381 and 0.688 -> 0.658 ms per iteration.  A fourth CTA per SM, 2 KB less
+// each, cost the mix's chains 0.66 -> 0.76: other chains' kernels no longer fit
+// beside them).
+template <typename R>
+__device__ __forceinline__ void put_sums(TriSmem<R> *tri, int slot, const TriSmem<R> &t) {
+  R4<R> *q = reinterpret_cast<R4<R> *>(tri + slot);
+  const int b = (slot >> 2) & 1;
+  q[b] = reinterpret_cast<const R4<R> *>(&t)[0];
+  q[b ^ 1] = reinterpret_cast<const R4<R> *>(&t)[1];
+}
+template <typename R>
+__device__ __forceinline__ TriSmem<R> get_sums(const TriSmem<R> *tri, int slot) {
+  const R4<R> *q = reinterpret_cast<const R4<R> *>(tri + slot);
+  const int b = (slot >> 2) & 1;
+  TriSmem<R> t;
+  reinterpret_cast<R4<R> *>(&t)[0] = q[b];
+  reinterpret_cast<R4<R> *>(&t)[1] = q[b ^ 1];
+  return t;
+}
+
 // Sums of one vertex's triangle terms in the order of its incidence list
 // (green_gauss.f:23-39 visits triangles in ascending order): entries
 // [j0, j1) of `vtl`, each a triangle slot and the vertex's position in it.
 // The slots and terms of up to B triangles are loaded before they are
 // added, so the shared-memory latency is paid once per B triangles; the
 // additions stay in list order (same bits as one triangle at a time).
-// vis = nullptr: inviscid (rv is zero).
-template <typename R, int B>
+// vis = nullptr: inviscid (rv is zero).  SWAP: records as put_sums writes them.
+template <typename R, int B, bool SWAP = false>
 __device__ __forceinline__ void grad_vertex_sums(const uint16_t *vtl, int j0, int j1,
                                                  const TriSmem<R> *tri, const R *vis, R qx[4],
                                                  R qy[4], R rv[3]) {
@@ -374,7 +399,10 @@ __device__ __forceinline__ void grad_vertex_sums(const uint16_t *vtl, int j0, in
     TriSmem<R> ts[B];
 #pragma unroll
     for (int u = 0; u < B; u++)
-      if (u < n) ts[u] = tri[e[u] & 0x3fff];
+      if (u < n) {
+        if constexpr (SWAP) ts[u] = get_sums<R>(tri, e[u] & 0x3fff);
+        else ts[u] = tri[e[u] & 0x3fff];
+      }
 #pragma unroll
     for (int u = 0; u < B; u++) {
       if (u < n) {
@@ -675,7 +703,7 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 
 #pragma unroll
           for (int j = 0; j < 3; j++) tri_visc_term<R>(tv, dbxx[j], dbyy[j], sv + 3 * j);
         }
-        s_tri[k] = ts;   // over this thread's own geometry entry
+        put_sums(s_tri, k, ts);   // over this thread's own geometry entry
       }
       __syncthreads();
       // phase 2: one thread per vertex, triangles in original order
@@ -684,8 +712,8 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRAD_MINB32 
         R qx[4], qy[4], rv[3];
         const int2 jr = s_vtr[threadIdx.x];
         // one triangle at a time: batched loads spill at 48 registers
-        grad_vertex_sums<R, 1>(s_vtl, jr.x - vt_a, jr.y - vt_a, s_tri, visc ? s_vis : nullptr, qx,
-                               qy, rv);
+        grad_vertex_sums<R, 1, true>(s_vtl, jr.x - vt_a, jr.y - vt_a, s_tri,
+                                     visc ? s_vis : nullptr, qx, qy, rv);
         const R ais = v_ais(A, v);
         Grad<R> g;
 #pragma unroll
