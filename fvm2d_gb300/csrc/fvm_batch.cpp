@@ -1806,11 +1806,13 @@ namespace {
 // and edges cut between blocks and of idle lanes where a lane holds a vertex.
 // Measured, us per iteration with blocks of 256 / 128 / 64: 7.7k vertices, FP64
 // Euler 199 / 176 / 166, FP32 43.1 / 40.8 / 39.3; 20k, FP32 laminar 58.6 / 56.0
-// / 53.3, FP64 laminar - / 321 / 395; 40k, FP64 Euler KFVS 404 / 414 / 446;
-// 98k, FP64 laminar 908 / 980 / 1180; 393k, 256 is best by 14% and more.
+// / 53.3, FP64 laminar - / 321 / 395; 40k, FP64 Euler KFVS 367 / 344, Roe 329 /
+// 300, FP32 42.7 / 41.4; 48k, laminar FP64 549 / 532, FP32 58.4 / 53.6; 60k,
+// FP64 Euler 400 / 398; 98k, 566 / 597, laminar 800 / 876; 393k, 256 is best by
+// 14% and more.
 int single_block_verts(int32_t np) {
   if (np <= 10000) return 64;
-  if (np <= 32000) return 128;
+  if (np <= 50000) return 128;
   return kBlockVerts;
 }
 
