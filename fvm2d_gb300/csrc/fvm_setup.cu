@@ -66,12 +66,17 @@ __global__ void k_fill(double *a, double v, int n) {
 // coordinates involved (rounding of a, p and the vector, and of the foot's
 // place along it); `off` and `e1.z` hold 3e-6 of the point's and the edge's.
 // `near` takes the distances of true candidates only (with bugcompat: the
-// first ends).  Infinite or NaN distances compare as "not farther".
+// first ends).  Infinite or NaN distances compare as "not farther".  Where
+// FP32 ends nothing is dropped: an edge or a point farther than kWallFar from
+// the origin (squares overflow) gets an infinite margin, and `near` is never
+// below kWallNear (squares underflow).  Far from zero the FP64 foot itself is
+// rounded (an ulp of the edge's coordinates): `e1.z` holds that too.
 // With every pair in FP64 (three roots and a quotient each) the pass took
 // 15.8 ms for 196,608 points and 768 edges; now 0.82 ms
 // (FP64 to FP32 conversions are as slow: with the edges' FP32 data formed by
 // every CTA instead of once, 1.77 ms).
 constexpr int kWallThreads = 128, kWallTile = 256, kWallList = 8;
+constexpr float kWallFar = 1e15f, kWallNear = 1e-12f;
 
 // squared distances to the candidates of one edge, folded into w
 __device__ __forceinline__ void wall_edge(double2 ci, double2 a, double2 b, int bugcompat,
@@ -107,11 +112,11 @@ __global__ void k_wall_edges(int nsedge, const double2 *__restrict__ coord,
   const float ax = (float)(a.x - org.x), ay = (float)(a.y - org.y);
   const float bx = (float)(b.x - org.x), by = (float)(b.y - org.y);
   const float dx = (float)(b.x - a.x), dy = bugcompat ? dx : (float)(b.y - a.y);
+  const float size = fabsf(ax) + fabsf(ay) + fabsf(bx) + fabsf(by) + fabsf(dx) + fabsf(dy);
+  float margin = 3e-6f * size + (float)(1e-15 * (fabs(a.x) + fabs(a.y) + fabs(b.x) + fabs(b.y)));
+  if (!(size <= kWallFar)) margin = __int_as_float(0x7f800000);
   edge32[2 * k] = make_float4(ax, ay, dx, dy);
-  edge32[2 * k + 1] = make_float4(1.0f / (dx * dx + dy * dy), bx,
-                                  3e-6f * (fabsf(ax) + fabsf(ay) + fabsf(bx) + fabsf(by) +
-                                           fabsf(dx) + fabsf(dy)),
-                                  by);
+  edge32[2 * k + 1] = make_float4(1.0f / (dx * dx + dy * dy), bx, margin, by);
 }
 
 __global__ void __launch_bounds__(kWallThreads) k_wall_dist(int np, int nsedge,
@@ -128,7 +133,8 @@ __global__ void __launch_bounds__(kWallThreads) k_wall_dist(int np, int nsedge,
   const double2 ci = (i < np) ? coord[i] : make_double2(0.0, 0.0);
   const double2 org = nsedge > 0 ? coord[sedge[0].x] : make_double2(0.0, 0.0);
   const float px = (float)(ci.x - org.x), py = (float)(ci.y - org.y);
-  const float off = 3e-6f * (fabsf(px) + fabsf(py));
+  const float size = fabsf(px) + fabsf(py);
+  const float off = size <= kWallFar ? 3e-6f * size : __int_as_float(0x7f800000);
   auto stage = [&](int t0) {
     __syncthreads();
     for (int k = threadIdx.x; k < kWallTile && t0 + k < nsedge; k += kWallThreads) {
@@ -156,7 +162,7 @@ __global__ void __launch_bounds__(kWallThreads) k_wall_dist(int np, int nsedge,
       near = fminf(near, sqrtf(d2) * 1.000001f + e1.z);
     }
   }
-  near += 2.f * off;
+  near = fmaxf(near + 2.f * off, kWallNear);
   double w = 1.0e20;   // (1e10)^2
   int n = 0;
   auto flush = [&]() {
