@@ -71,17 +71,26 @@ inline cudaError_t launch_grad_f64(const ArenaPtrs<R> &A, const LaunchCfg &c, in
   }
   return cudaGetLastError();
 }
+// What a kernel may take of dynamic shared memory is a property of the function
+// in the whole process, so it is set to all that its static part leaves, whatever
+// this batch needs: set to a batch's own need, a smaller batch or handle created
+// later took it from a larger one, whose next launch then failed.
+template <typename K>
+inline cudaError_t allow_smem(K kern, size_t need) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+  if (e != cudaSuccess) return e;
+  const size_t most = kMaxSmem - a.sharedSizeBytes;
+  if (need > most) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 template <typename R>
 inline cudaError_t grad_attributes(size_t sm) {
-  cudaError_t e = cudaFuncSetAttribute(k_grad<KT<R>, 0>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  cudaError_t e = allow_smem(k_grad<KT<R>, 0>, sm);
   if constexpr (sizeof(R) == 8) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_grad<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sm);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_grad<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sm);
+    if (e == cudaSuccess) e = allow_smem(k_grad<KT<R>, 1>, sm);
+    if (e == cudaSuccess) e = allow_smem(k_grad<KT<R>, 2>, sm);
   }
   return e;
 }
@@ -139,20 +148,18 @@ inline void launch_flux_any(const ArenaPtrs<R> &A, const LaunchCfg &c, int stage
 // Dynamic shared memory of the FP32 flux kernels (FP64: none).
 template <typename R>
 inline cudaError_t flux_attributes(size_t f) {
+  cudaError_t e = cudaSuccess;
   if constexpr (sizeof(R) == 4) {
-    const int b = (int)f;
-    cudaError_t e = cudaFuncSetAttribute(k_flux<KT<R>, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 1 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 2 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux<KT<R>, 3 | kFluxStd>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    return e;
-  } else {
-    return cudaSuccess;
+    e = allow_smem(k_flux<KT<R>, 0>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 1>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 2>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 3>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, kFluxStd>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 1 | kFluxStd>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 2 | kFluxStd>, f);
+    if (e == cudaSuccess) e = allow_smem(k_flux<KT<R>, 3 | kFluxStd>, f);
   }
+  return e;
 }
 
 #define FVM_DEFINE_LAUNCHERS(R)                                                            \
@@ -304,29 +311,21 @@ inline cudaError_t flux_attributes(size_t f) {
     const size_t st = smem_step(c, (R *)nullptr);                                          \
     if (g > kMaxSmem || f > kMaxSmem || s > kMaxSmem || st > kMaxSmem)                     \
       return cudaErrorInvalidConfiguration;                                                \
-    for (int k = 0; k < 4; k++) {                                                          \
-      cudaError_t e2 = cudaSuccess;                                                        \
-      if (k == 0) e2 = cudaFuncSetAttribute(k_step<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
-      if (k == 1) e2 = cudaFuncSetAttribute(k_step<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
-      if (k == 2) e2 = cudaFuncSetAttribute(k_step<R, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
-      if (k == 3) e2 = cudaFuncSetAttribute(k_step<R, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st); \
-      if (e2 != cudaSuccess) return e2;                                                    \
-    }                                                                                      \
-    cudaError_t e = grad_attributes<R>(g);                                                 \
+    cudaError_t e = allow_smem(k_step<R, 0>, st);                                          \
+    if (e == cudaSuccess) e = allow_smem(k_step<R, 1>, st);                                \
+    if (e == cudaSuccess) e = allow_smem(k_step<R, 2>, st);                                \
+    if (e == cudaSuccess) e = allow_smem(k_step<R, 3>, st);                                \
+    if (e == cudaSuccess) e = grad_attributes<R>(g);                                       \
     if (e == cudaSuccess) e = flux_attributes<R>(f);                                       \
-    if (e == cudaSuccess)                                                                  \
-      e = cudaFuncSetAttribute(k_sa<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s); \
+    if (e == cudaSuccess) e = allow_smem(k_sa<KT<R>>, s);                                  \
+    const size_t ge = size_t(c.max_slots) * sizeof(Grad<R>);                               \
     const size_t gb = grad_bulk_layout(c.max_tri, kTriLocMax, c.viscous).total;            \
+    /* (where these two do not fit, their launchers say so) */                             \
+    if (e == cudaSuccess && ge <= kMaxSmem) e = allow_smem(k_gradient_edge<KT<R>>, ge);    \
     if (e == cudaSuccess && sizeof(R) == 4 && gb <= kMaxSmem)                              \
-      e = cudaFuncSetAttribute(k_grad_bulk<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gb); \
-    const size_t ge = size_t(c.max_slots) * sizeof(Grad<R>);                                 \
-    if (e == cudaSuccess && ge <= kMaxSmem)                                                \
-      e = cudaFuncSetAttribute(k_gradient_edge<KT<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ge); \
-    const int pmax = (int)(kMaxSmem - kPipeStaticSmem);                                    \
-    if (e == cudaSuccess && sizeof(R) == 4)                                                \
-      e = cudaFuncSetAttribute(k_grad_pipe<KT<R>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
-    if (e == cudaSuccess && sizeof(R) == 4)                                                \
-      e = cudaFuncSetAttribute(k_grad_pipe<KT<R>, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, pmax); \
+      e = allow_smem(k_grad_bulk<KT<R>>, gb);                                              \
+    if (e == cudaSuccess && sizeof(R) == 4) e = allow_smem(k_grad_pipe<KT<R>, 1>, 0);      \
+    if (e == cudaSuccess && sizeof(R) == 4) e = allow_smem(k_grad_pipe<KT<R>, 2>, 0);      \
     return e;                                                                              \
   }
 
