@@ -178,7 +178,7 @@ struct MeshCtl {
 };
 
 struct BlockPartial {       // conres.f:14-22 partials of one block
-  double sumsq;
+  double sumsq;             // (FP32 states, a split leaf: the bits of a pair of floats)
   double maxabs;
   int argmax;               // driver index (1-based); INT_MAX if none
   int pad;

@@ -908,14 +908,15 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_GRADV_MINB32
 // of the CTA (contains barriers).  FP64 states: FP64 arithmetic as before.
 // FP32 states: gra is formed exactly as a pair of floats (TwoSum), its
 // square as a pair (FMA residual), and the warp and block sums are pair
-// sums, converted to FP64 once per block.  The FP64 pipe of this GPU is
-// slow, and this keeps it out of the reduction: the sum carries ~2^-47
-// relative error instead of 2^-53; max |gra| is exact.
+// sums, converted to FP64 once per leaf: by the block, or, where the leaf is
+// split into several, by the monitor from their pairs (`split`).  The FP64
+// pipe of this GPU is slow, and this keeps it out of the reduction: the sum
+// carries ~2^-47 relative error instead of 2^-53; max |gra| is exact.
 // ---------------------------------------------------------------------------
 // The sums of a block's eight warps (32 consecutive vertices each) are added
 // in pairs, and a mesh whose leaves of 256 vertices are split into smaller
-// blocks adds those blocks' records in the same pairs (conres_block), so the
-// norm does not depend on the split.
+// blocks adds those blocks' records in the same pairs and the same arithmetic
+// (conres_share), so the norm does not depend on the split.
 static_assert(kBlockVerts == 256, "eight warps");
 __device__ __forceinline__ double warp_sums(const double *s) {
   return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
@@ -942,7 +943,7 @@ __device__ __forceinline__ bool df_greater(DFloat x, DFloat y) {   // normalized
 template <typename R>
 __device__ __forceinline__ void block_conres_partial(bool have, R rho_new, R rho_old, int orig,
                                                      double *s_red, double *s_max, int *s_arg,
-                                                     BlockPartial *out) {
+                                                     BlockPartial *out, bool split) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int darg = INT_MAX;
   if constexpr (sizeof(R) == 8) {
@@ -1016,7 +1017,8 @@ __device__ __forceinline__ void block_conres_partial(bool have, R rho_new, R rho
         }
       }
       BlockPartial bp;
-      bp.sumsq = double(t.hi) + double(t.lo);
+      bp.sumsq = split ? __hiloint2double(__float_as_int(t.hi), __float_as_int(t.lo))
+                       : double(t.hi) + double(t.lo);
       bp.maxabs = double(m.hi) + double(m.lo);   // exact
       bp.argmax = a;
       bp.pad = 0;
@@ -1523,7 +1525,8 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
     }
   }
   if (mode == MODE_UPDATE && stage == 3)
-    block_conres_partial<R>(have, rho_new, rho_old, org, s_red, s_max, s_arg, A.part + bi.part);
+    block_conres_partial<R>(have, rho_new, rho_old, org, s_red, s_max, s_arg, A.part + bi.part,
+                            mc.sub > 1);
 }
 
 // FP64 flux pass, first kernel: the flux of every edge once, into eflux (the
@@ -1949,7 +1952,8 @@ __global__ void __launch_bounds__(kBlockVerts, sizeof(R) == 4 ? FVM_FLUX_MINB32 
       }
     }
     if (stage == 3)
-      block_conres_partial<R>(have, rho_new, rho_old, org, s_red, s_max, s_arg, A.part + bi.part);
+      block_conres_partial<R>(have, rho_new, rho_old, org, s_red, s_max, s_arg, A.part + bi.part,
+                              mc.sub > 1);
     __syncthreads();
   }
 }
@@ -2216,8 +2220,26 @@ __device__ __forceinline__ void reduce_force(Moments &v) {
 // A thread's share of a mesh's conres partials: thread t of n.  The partials
 // are contiguous (block k's record is blk0 + k); eight loads in flight per
 // thread (a 2048-block mesh in one trip): the records of 8 / sub leaves, each
-// leaf's `sub` records added in pairs and the leaves in order.
-template <typename R>
+// leaf's `sub` records added in pairs and the leaves in order.  PAIRS: the
+// records of split leaves hold float pairs (block_conres_partial of FP32 states),
+// added as a block of the whole leaf adds its warps.
+__device__ __forceinline__ DFloat pair_of(const BlockPartial &p) {
+  return {__int_as_float(__double2hiint(p.sumsq)), __int_as_float(__double2loint(p.sumsq))};
+}
+template <bool PAIRS>
+__device__ __forceinline__ double leaf_sum2(const BlockPartial *p) {
+  if constexpr (!PAIRS) return p[0].sumsq + p[1].sumsq;
+  const DFloat t = df_add(pair_of(p[0]), pair_of(p[1]));
+  return double(t.hi) + double(t.lo);
+}
+template <bool PAIRS>
+__device__ __forceinline__ double leaf_sum4(const BlockPartial *p) {
+  if constexpr (!PAIRS) return (p[0].sumsq + p[1].sumsq) + (p[2].sumsq + p[3].sumsq);
+  const DFloat t = df_add(df_add(pair_of(p[0]), pair_of(p[1])),
+                          df_add(pair_of(p[2]), pair_of(p[3])));
+  return double(t.hi) + double(t.lo);
+}
+template <typename R, bool PAIRS>
 __device__ __forceinline__ void conres_share(const ArenaPtrs<R> &A, const MeshConst &mc, int t,
                                              int n, Moments &v) {
   constexpr int kU = 8;
@@ -2231,12 +2253,12 @@ __device__ __forceinline__ void conres_share(const ArenaPtrs<R> &A, const MeshCo
       else bp[u] = BlockPartial{0.0, 0.0, INT_MAX, 0};
     }
     if (sub == 4) {
-      v.s += (bp[0].sumsq + bp[1].sumsq) + (bp[2].sumsq + bp[3].sumsq);
-      if (i0 + n < nleaf) v.s += (bp[4].sumsq + bp[5].sumsq) + (bp[6].sumsq + bp[7].sumsq);
+      v.s += leaf_sum4<PAIRS>(bp);
+      if (i0 + n < nleaf) v.s += leaf_sum4<PAIRS>(bp + 4);
     } else if (sub == 2) {
 #pragma unroll
       for (int u = 0; u < kU; u += 2)
-        if (i0 + u / 2 * n < nleaf) v.s += bp[u].sumsq + bp[u + 1].sumsq;
+        if (i0 + u / 2 * n < nleaf) v.s += leaf_sum2<PAIRS>(bp + u);
     } else {
 #pragma unroll
       for (int u = 0; u < kU; u++)
@@ -2281,13 +2303,13 @@ __device__ __forceinline__ void force_share(const ArenaPtrs<float> &A, const Mes
 }
 
 // The monitor's reduction, by all kMonitorMaxThreads threads (`what`: 1 the
-// residual, 2 the force, 3 both).  Warp 0 returns the residual's part and
-// warps 1 and 2 the force.  One CTA does this between two iterations, so its
+// residual, 2 the force, 3 both; PAIRS: see conres_share).  Warp 0 returns the
+// residual's part and warps 1 and 2 the force.  One CTA does this between two iterations, so its
 // latency counts and an FP64 operation of a warp costs 64 cycles: comparisons
 // read the bits, each reduction is five shuffles and one exchange, and the
 // final scalars are formed by different warps.  8 x 1024x384, alone, 22.4 us
 // as two 8-level shared-memory trees with one thread finishing; now 16.3 us (160 x 48: 9.6, now 5.2).
-template <typename R>
+template <typename R, bool PAIRS>
 __device__ __forceinline__ Moments mesh_moments(const ArenaPtrs<R> &A, const MeshConst &mc,
                                                 const R4<R> *P, int what) {
   __shared__ Moments s_w[kMonitorMaxThreads / 32];
@@ -2295,7 +2317,7 @@ __device__ __forceinline__ Moments mesh_moments(const ArenaPtrs<R> &A, const Mes
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Moments v = {0.0, 0.0, 0.0, 0.0, INT_MAX};
   if constexpr (sizeof(R) == 4) {
-    if (what & 1) conres_share<R>(A, mc, threadIdx.x, kMonitorMaxThreads, v);
+    if (what & 1) conres_share<R, PAIRS>(A, mc, threadIdx.x, kMonitorMaxThreads, v);
     if (what & 2) {
       force_share(A, mc, P, threadIdx.x, kMonitorMaxThreads, v);
       reduce_force<32>(v);
@@ -2318,7 +2340,7 @@ __device__ __forceinline__ Moments mesh_moments(const ArenaPtrs<R> &A, const Mes
           f = force_chain(s_f[i & 1], lane, min(mc.nsw - i * kForceTile, kForceTile), viscous, f);
       } else {
         if (i == 0 && (what & 1))
-          conres_share<R>(A, mc, threadIdx.x - 32, kMonitorMaxThreads - 32, v);
+          conres_share<R, PAIRS>(A, mc, threadIdx.x - 32, kMonitorMaxThreads - 32, v);
         if (i + 1 < nt) {
           const int base = (i + 1) * kForceTile, n = min(mc.nsw - base, kForceTile);
           for (int k = threadIdx.x - 32; k < n; k += kMonitorMaxThreads - 32)
@@ -2369,7 +2391,7 @@ __global__ void __launch_bounds__(kMonitorMaxThreads) k_monitor(ArenaPtrs<R> A) 
   // the control block is read here and written after the reduction's barrier
   const int err = ctl.err, err_point = ctl.err_point;
   const int row = ctl.hist_off + ctl.n_done % ctl.hist_cap;
-  const Moments v = mesh_moments<R>(A, mc, A.st[newp], 3);
+  const Moments v = mesh_moments<R, sizeof(R) == 4>(A, mc, A.st[newp], 3);
   const bool stopped = err != 0 || err_point != INT_MAX;
   if (threadIdx.x == 32 && !stopped) {
     const double cl = force_coefficient(mc, v, 0);
@@ -2529,7 +2551,8 @@ __global__ void __launch_bounds__(kMonitorMaxThreads)
     k_routine_monitor(ArenaPtrs<R> A, int mesh, int what, int first) {
   MeshCtl &ctl = A.ctl[mesh];
   const MeshConst &mc = A.mc[mesh];
-  const Moments v = mesh_moments<R>(A, mc, A.st[ctl.phase], what == 0 ? 1 : 2);
+  // (k_conres_part sums in FP64 for either precision)
+  const Moments v = mesh_moments<R, false>(A, mc, A.st[ctl.phase], what == 0 ? 1 : 2);
   if (what == 0) {
     if (threadIdx.x != 0) return;
     double fres = residual_norm(mc, v);
