@@ -10,6 +10,7 @@
 //   routine mode (stage 0): state = p, prim_old = p+2, updates in place.
 #pragma once
 
+#include <cfloat>
 #include <climits>
 
 #include "fvm_device.cuh"
@@ -983,6 +984,9 @@ __device__ __forceinline__ void block_conres_partial(bool have, R rho_new, R rho
       mx = g.hi >= 0.f ? g : DFloat{-g.hi, -g.lo};
       if (mx.hi > 0.f) darg = orig;
       else mx = DFloat{0.f, 0.f};   // NaN or no change (see the FP64 branch)
+      // (TwoSum's low part of an infinite change is NaN; max_first needs a
+      // number, and equal maxima compare equal only with equal low parts)
+      if (mx.hi > FLT_MAX) mx.lo = 0.f;
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
