@@ -302,7 +302,9 @@ inline cudaError_t flux_attributes(size_t f) {
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_limitgrad(const ArenaPtrs<R> &A, const LaunchCfg &c) {                 \
-    k_limitgrad<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                               \
+    /* the hardware's operations: F64's called quotients made 98k vertices 75 us */        \
+    /* a call instead of 67, 1.2k vertices 27 instead of 23 */                             \
+    k_limitgrad<R><<<c.grid, kBlockVerts, 0, c.stream>>>(A);                               \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t prepare_attributes(const LaunchCfg &c, R *) {                                \
