@@ -242,9 +242,15 @@ FVM_I64 bool pos64(double a) {
 FVM_I64_CALL double i64_mul_call(double a, double b) { return mul64(a, b); }
 FVM_I64_CALL double i64_div_call(double a, double b) { return div64(a, b); }
 FVM_I64_CALL double i64_sqrt_call(double a) { return sqrt64(a); }
+// FVM_FP64_CONTRACT (the library with contracted FP64 kernels): products on the
+// FP64 pipe in every form, where the compiler can join them with sums.
 template <int C>
 FVM_I64 double mul_as(double a, double b) {
+#ifdef FVM_FP64_CONTRACT
+  return a * b;
+#else
   return C == 2 ? a * b : C ? i64_mul_call(a, b) : mul64(a, b);
+#endif
 }
 template <int C>
 FVM_I64 double div_as(double a, double b) { return C ? i64_div_call(a, b) : div64(a, b); }
