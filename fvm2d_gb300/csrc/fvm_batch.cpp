@@ -1785,6 +1785,13 @@ extern "C" int32_t fvm_layout_stats(const fvm_mesh *m, int64_t *out) {
   out[7] = L.max_loc;
   out[8] = (int64_t)L.halo_ids.size();
   out[9] = verify_layout(L);
+  // the layouts of the other precision and of small single meshes
+  for (int bv = kBlockVerts; bv >= kBlockVerts / 4; bv /= 2)
+    for (const bool fp64 : {true, false}) {
+      if (fp64 && bv == kBlockVerts) continue;   // above
+      if ((st = build_layout(*m, bv, fp64, L))) return st;
+      out[9] += verify_layout(L);
+    }
   return FVM_OK;
 }
 

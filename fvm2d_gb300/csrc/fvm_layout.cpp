@@ -441,6 +441,12 @@ int64_t verify_layout(const MeshLayout &L) {
     if (L.neo.size() != L.blocks.size() || L.neo[b] < 0 || L.neo[b] > bi.ne) return 1;
     std::fill(owned.begin() + bi.e0, owned.begin() + bi.e0 + L.neo[b], 1);
   }
+  // `sub` consecutive blocks make a leaf of kBlockVerts vertices (the monitor
+  // adds their residual records as one leaf's)
+  const int bv = kBlockVerts / std::max(L.sub, 1);
+  if (L.sub < 1 || (int)L.blocks.size() != L.nblk || L.nblk != (L.np + bv - 1) / bv) return 1;
+  for (int b = 0; b < L.nblk; b++)
+    if (L.blocks[b].v0 != b * bv || L.blocks[b].nv != std::min(bv, L.np - b * bv)) bad++;
   auto has = [](const int4 &t, int v, int pos) {
     return (pos == 0 ? t.x : pos == 1 ? t.y : t.z) == v;
   };

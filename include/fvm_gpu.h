@@ -500,13 +500,15 @@ int32_t fvm_serve_times(fvm_server *s, double *out);
  * on this server may start once destroy has been called. */
 int32_t fvm_serve_destroy(fvm_server *s);
 
-/* Layout statistics of a mesh after renumbering (no GPU needed):
+/* Layout statistics of a mesh after renumbering (no GPU needed), of the
+ * layout an FP64 batch gives it:
  * out[0] blocks, [1] interior edge entries (cut edges counted in both
  * blocks), [2] triangle entries (block and halo), [3] max slots of a
  * block, [4] max triangles of a block, [5] boundary edge entries, [6] max
  * triangles of a block and its halo, [7] max own + halo vertices, [8] halo
- * vertices, [9] violations of the layout's invariants (0 for a valid
- * layout).  out has 10 elements. */
+ * vertices, [9] violations of the invariants of this and of every other
+ * layout a mesh can get (FP32, blocks of 128 and 64; 0 for valid layouts).
+ * out has 10 elements. */
 int32_t fvm_layout_stats(const fvm_mesh *m, int64_t *out);
 
 #ifdef __cplusplus
