@@ -129,6 +129,8 @@ SIGNATURES = {
     "fvm_batch_timing_read": (C.c_int32, [C.c_void_p, C.c_int32, C.c_char_p, _pd,
                                           C.POINTER(C.c_int64), _pi]),
     "fvm_batch_launch_count": (C.c_int64, [C.c_void_p]),
+    "fvm_batch_edge_form": (C.c_int32, [C.c_void_p]),
+    "fvm_gpu_edge_form": (C.c_int32, [C.c_void_p]),
     "fvm_batch_test_wait_timeout": (C.c_int32, [C.c_void_p, C.c_int64]),
     "fvm_gpu_gradient": (C.c_int32, [C.c_void_p]),
     "fvm_gpu_shockind": (C.c_int32, [C.c_void_p]),

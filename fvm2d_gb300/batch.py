@@ -205,6 +205,10 @@ class Batch:
     def launch_count(self) -> int:
         return int(L.lib().fvm_batch_launch_count(self.h))
 
+    def edge_form(self) -> int:
+        """Form of the FP64 edge pass for the resident meshes (fvm_batch_edge_form)."""
+        return int(L.lib().fvm_batch_edge_form(self.h))
+
     TUNE_CANDIDATES = ("bulk", "loads", "vertex", "fused", "split+overlap", "fused+overlap",
                        "split+overlap4", "split+overlap8", "pipe", "pipe+overlap",
                        "pipe+overlap4")

@@ -1755,6 +1755,10 @@ extern "C" int32_t fvm_batch_timing_read(fvm_batch *b, int32_t max, char *names,
 
 extern "C" int64_t fvm_batch_launch_count(fvm_batch *b) { return b ? b->launches : -1; }
 
+extern "C" int32_t fvm_batch_edge_form(fvm_batch *b) {
+  return b && b->prec == FVM_PREC_FP64 ? b->cfg.edge_form : -1;
+}
+
 extern "C" int32_t fvm_batch_test_wait_timeout(fvm_batch *b, int64_t budget_cycles) {
   if (b && b->pending) {   // deferred admissions first
     const int32_t cst = batch_commit(b);
@@ -1978,6 +1982,8 @@ extern "C" int32_t fvm_gpu_time_step(fvm_handle *h) {
   FVM_TRY(b, cudaStreamSynchronize(b->stream));
   return FVM_OK;
 }
+
+extern "C" int32_t fvm_gpu_edge_form(fvm_handle *h) { return h ? fvm_batch_edge_form(h->b) : -1; }
 
 extern "C" int32_t fvm_gpu_residu(fvm_handle *h) {
   if (!h) return FVM_ERR_ARG;

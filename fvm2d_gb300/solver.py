@@ -198,6 +198,10 @@ class Solver:
         check(L.lib().fvm_gpu_get_prim_old(self.h, dptr(r)), "fvm_gpu_get_prim_old")
         return r
 
+    def edge_form(self) -> int:
+        """Form of the FP64 edge pass for this mesh (fvm_gpu_edge_form)."""
+        return int(L.lib().fvm_gpu_edge_form(self.h))
+
     # ---- routines of main.f:44-62 -------------------------------------------
     def save_old(self):
         check(L.lib().fvm_gpu_save_old(self.h), "save_old")

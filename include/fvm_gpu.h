@@ -391,6 +391,12 @@ int32_t fvm_batch_timing_read(fvm_batch *b, int32_t max, char *names,
                               double *ms, int64_t *launches, int32_t *n);
 /* Launches of this library's kernels since the batch was created. */
 int64_t fvm_batch_launch_count(fvm_batch *b);
+/* The form of the FP64 edge pass that the resident meshes' number of edges
+ * chooses (every form gives the same bits): 0 a thread per edge, 1 the same
+ * with called operations, for many edges, 2 four warps to 32 edges, for few;
+ * -1 for an FP32 batch.  fvm_gpu_edge_form: of a handle. */
+int32_t fvm_batch_edge_form(fvm_batch *b);
+int32_t fvm_gpu_edge_form(fvm_handle *h);
 /* Test of the bounded device waits (no counterpart in the reference): one
  * stage-1 gradient pass of the pipelined kernel (FP32 batches) in which the
  * first block of every CTA is armed for its copies but the copies are never
