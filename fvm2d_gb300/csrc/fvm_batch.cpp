@@ -550,7 +550,10 @@ int32_t update_work(fvm_batch *b) {
   // CTAs (4 x 128 per SM), where a warp's own latency counts; called above,
   // where the warps wait for instructions.  us per iteration, inlined / called:
   // 23k vertices (69k edges) Roe 219 / 254; 40k (119k edges) Roe 347 / 337, KFVS
-  // 404 / 387, HLLC 662 / 606; 98k laminar 901 / 871; 393k Roe 2417 / 2096.
+  // 404 / 387, HLLC 662 / 606; 98k laminar 901 / 871; 393k Roe 2417 / 2096;
+  // three meshes of one solver each (the kernel that holds all three, whose
+  // spills at seven CTAs cost less than they give) 3 x 23k 817 / 783, 3 x 98k
+  // 3200 / 2441.
   // Few edges, the items of four warps to 32 edges in one wave (6 CTAs per SM):
   // a variable to a warp and products on the FP64 pipe.  us per iteration, thread
   // per edge / four warps: 1.5k vertices Roe 136 / 105, KFVS 137 / 109; 7.7k Roe

@@ -356,11 +356,11 @@ __device__ __forceinline__ void tri_visc_term(const TriVisc<R> &tv, R dbx, R dby
 // FP32 triangle sums in shared memory, the record's two 16-byte halves swapped
 // where bit 2 of the slot is set: neighbouring threads read slots one or two
 // apart, whose like halves would share a quarter or half of the banks (60% of
-// the gradient's shared-memory wavefronts were conflicts; 4 x 768x256 turbulent
-// 0.072 -> 0.064 ms per stage, the 24-mesh mix 0.132 -> 0.122, and 0.399 ->
-// 0.381 and 0.688 -> 0.658 ms per iteration.  A fourth CTA per SM, 2 KB less
-// each, cost the mix's chains 0.66 -> 0.76: other chains' kernels no longer fit
-// beside them).
+// the gradient's shared-memory wavefronts were conflicts, now 45%; 4 x 768x256
+// turbulent 0.072 -> 0.064 ms per stage, the 24-mesh mix 0.132 -> 0.122, and
+// 0.399 -> 0.381 and 0.688 -> 0.658 ms per iteration.  A fourth CTA per SM, 2
+// KB less each, cost the mix's chains 0.66 -> 0.76: other chains' kernels no
+// longer fit beside them).
 template <typename R>
 __device__ __forceinline__ void put_sums(TriSmem<R> *tri, int slot, const TriSmem<R> &t) {
   R4<R> *q = reinterpret_cast<R4<R> *>(tri + slot);
@@ -1162,8 +1162,9 @@ __device__ __forceinline__ F2 limit_albada2(F2 ul, F2 ur, F2 ur2, F2 eps) {
 // the limiter, albada21 scales the edge vector once per edge instead of each
 // projected gradient, and albada22 * dq serves both sides; the same values as
 // recon1 up to FP32 rounding.  The pass is bound by issue and latency together
-// (48% issue over a launch): pairs take a third off the reconstruction's
-// instructions, 8 x 1024x384 0.1785 -> 0.1697 ms per launch alone.
+// (63% issue-active, 53% over a whole launch): pairs take a third off the
+// reconstruction's instructions, 8 x 1024x384 0.1785 -> 0.1697 ms per launch
+// alone.
 __device__ __forceinline__ void recon_edge_f32(const R4<float> &p1, const R4<float> &p2,
                                                const Grad<float> &g1, const Grad<float> &g2,
                                                float dx, float dy, const FluxConst<float> &fc,
@@ -1547,8 +1548,11 @@ __device__ __forceinline__ void flux_gather(const ArenaPtrs<R> &A, const MeshCon
 // instructions, of which one edge takes 5800 (93 KB).  C = 1 calls the
 // operations instead of inlining them, and few live values (the reconstructed
 // states and the central flux wait in shared memory) let seven CTAs share an
-// SM: 442 us; the rule is in update_work.  HLLC on 768 x 256: 1064 -> 560 us,
-// 390 us since its pow are shared out (edge_hllc_star).
+// SM: 442 us (FP64 77%, ALU 46%, issue 55%); the rule is in update_work.  HLLC
+// on 768 x 256: 1064 -> 560 us, 390 us since its pow are shared out
+// (edge_hllc_star).  Zeros lie outside the integer operations' window: where the
+// flow is still uniform the differences take the hardware's, and the pass of
+// the first iterations from freestream lasts 670 us (FP64 80%, issue 41%).
 template <typename R, int FLUX, int C>
 __global__ void __launch_bounds__(kEdgeThreads, C == 2   ? FVM_EFLUX_FEWB
                                                 : C == 1 ? FVM_EFLUX_CALLB
@@ -2135,7 +2139,7 @@ __device__ __forceinline__ void wall_force(float2 sv, float mu1, float mu2,
 // and form the next tile.  Each addition costs one pass through the FP64 pipe (about 32 ns on
 // this GPU, 2 lanes per SM quarter-cycle), which bounds the chain: with the
 // loads and products of every edge inside it the chain took 1.45 ms for 1024
-// edges, k_monitor 1480 us against FORCE_US us now.  mu = 0 (inviscid meshes)
+// edges, k_monitor 1480 us; now 49 us.  mu = 0 (inviscid meshes)
 // makes both viscous terms zero; subtracting zero changes no sum (it never is
 // -0: it starts at +0), so a tile whose viscous terms all are zero adds the
 // pressure terms alone.  NaN terms count as nonzero.

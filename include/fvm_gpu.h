@@ -291,7 +291,12 @@ int32_t fvm_gpu_conres_noalloc(const double *prim, const double *prim_old,
 typedef struct fvm_batch fvm_batch;
 
 typedef struct fvm_batch_caps {
-  int64_t vertices;          /* total vertices of all resident meshes         */
+  int64_t vertices;          /* total vertices of all resident meshes; with
+                                the derived capacities below an arena takes
+                                about 940 bytes of device memory for each in
+                                FP64 (164 of them the edge fluxes between
+                                the two kernels of the flux pass), 745 in
+                                FP32 (fvm_prepared_bytes: of one mesh)       */
   int32_t meshes;            /* resident meshes at a time                     */
   int32_t viscous;           /* 1 if laminar/turbulent meshes may be admitted */
   /* optional overrides; 0 = derived from vertices and meshes */
