@@ -42,6 +42,7 @@ constexpr int kTriPosShift = 14;           // triangle entry: vertex position 0.
 // per-vertex flag bits
 constexpr uint8_t kVtxSolid = 1;
 constexpr uint8_t kVtxFarfield = 2;
+constexpr uint8_t kVtxShock = 4;   // between the two kernels of shockind.f
 
 struct BlockInfo {          // 16 ints, one per CTA
   int mesh;                 // mesh slot
@@ -232,7 +233,7 @@ struct ArenaPtrs {
   const double *ais;     // (1/6)/mcarea
   const double *cvarea, *drmin, *wd;
   const int *orig;       // driver index (1-based) of each vertex
-  const uint8_t *vflag;
+  uint8_t *vflag;
   // incidence: per vertex {begin, end} into the list arrays
   const int2 *ve_rng;
   const uint16_t *ve_list;

@@ -2674,8 +2674,9 @@ __global__ void __launch_bounds__(kBlockVerts) k_gradient_edge(ArenaPtrs<R> A) {
 // shockind.f:1-52 (never called by the reference), routine mode: the
 // density-jump indicator of every vertex from all its edges (edge order),
 // ind/drmin/cvarea**0.75; the gradients of vertices where it exceeds 1 are
-// set to zero.  One thread per vertex; each edge's term is formed by both
-// of its ends with the same operations, so both add the same value.
+// set to zero, by a second kernel: the first reads its neighbours' gradients.
+// One thread per vertex; each edge's term is formed by both of its ends with
+// the same operations, so both add the same value.
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(kBlockVerts) k_shockind(ArenaPtrs<R> A) {
@@ -2711,12 +2712,23 @@ __global__ void __launch_bounds__(kBlockVerts) k_shockind(ArenaPtrs<R> A) {
       ind = ind + li;
     }
     ind = ind / v_drmin(A, v) / mpow(v_cvarea(A, v), R(0.75));
-    if (ind > R(1)) {
-      Grad<R> z;
+    const uint8_t f = A.vflag[v];
+    A.vflag[v] = ind > R(1) ? f | kVtxShock : f & (uint8_t)~kVtxShock;
+  }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kBlockVerts) k_shock_zero(ArenaPtrs<R> A) {
+  int w0, nwork;
+  work_range(A, w0, nwork);
+  for (int w = w0 + blockIdx.x; w < nwork; w += gridDim.x) {
+    const BlockInfo bi = work_block(A, w);
+    const int v = bi.v0 + threadIdx.x;
+    if (threadIdx.x >= bi.nv || !(A.vflag[v] & kVtxShock)) continue;
+    Grad<R> z;
 #pragma unroll
-      for (int q = 0; q < 4; q++) z.qx[q] = z.qy[q] = R(0);
-      A.grad[v] = z;
-    }
+    for (int q = 0; q < 4; q++) z.qx[q] = z.qy[q] = R(0);
+    A.grad[v] = z;
   }
 }
 

@@ -299,6 +299,7 @@ inline cudaError_t flux_attributes(size_t f) {
   }                                                                                        \
   cudaError_t launch_shockind(const ArenaPtrs<R> &A, const LaunchCfg &c) {                  \
     k_shockind<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                                \
+    k_shock_zero<KT<R>><<<c.grid, kBlockVerts, 0, c.stream>>>(kptrs(A));                   \
     return cudaGetLastError();                                                             \
   }                                                                                        \
   cudaError_t launch_limitgrad(const ArenaPtrs<R> &A, const LaunchCfg &c) {                 \
