@@ -610,7 +610,8 @@ def serving(args):
                   "request's own stop), one solve at a time, wall clock, on the served requests "
                   f"at the size quantiles (2i+1)/{2 * k}; solves/s = sample size / total seconds; "
                   "fp64_strict: no FMA contraction (bitwise the reference's arithmetic), "
-                  "fp64_fma: the same kernels with FMA contraction")
+                  "fp64_fma: the library with products on the FP64 pipe and FMA "
+                  "contraction allowed")
     vs["sample"] = [{"rid": r.rid, "vertices": r.npts, "laminar": r.laminar} for r in sample]
     out["vs_fp64_gpu"] = vs
     rows = []

@@ -428,7 +428,8 @@ int32_t fvm_batch_test_wait_timeout(fvm_batch *b, int64_t budget_cycles);
  * iteration (0 for a candidate that does not fit), *choice the candidate
  * kept: 0 bulk, 1 loads, 2 per vertex, 3 fused, 4 bulk (FP32) or loads
  * (FP64) in two overlapped chains, 5 fused in two chains, 6 and 7 as 4 in
- * four and eight chains. */
+ * four and eight chains, 8 the pipelined gradient (FP32), 9 and 10 the same
+ * in two and four chains. */
 int32_t fvm_batch_tune(fvm_batch *b, int32_t iters, int32_t max, double *ms_per_iter,
                        int32_t *choice);
 /* Sets the form of the iteration to a candidate of fvm_batch_tune (the
